@@ -15,23 +15,6 @@ struct alignas(16) bf16x8 {
   uint32_t u[4];
 };
 
-__device__ __forceinline__ float block_sum_128(float v, float* red) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  return red[0] + red[1] + red[2] + red[3];
-}
-__device__ __forceinline__ float block_max_128(float v, float* red) {
-  v = warp_max(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  return fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
-}
-
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
   // satfinite conversion; inputs are already scaled into [-448, 448].
   __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
@@ -58,8 +41,7 @@ __device__ __forceinline__ float row_scale_from_amax(float amax, float qmax) {
 // is processed: thread t copies its own 16-byte vectors (t, t+T, t+2T, ...) of a row into a slot of a shared-memory
 // ring with cp.async and later reads exactly those vectors back itself, so the ring needs no barrier - only
 // cp.async.wait_group.  Measured at 32760 x 5120: 146 -> 107 us (3.4 -> 4.7 TB/s).  The LayerNorm and RMSNorm kernels
-// keep one row per CTA: they are bound by instruction issue (fp32 math on bf16 data plus per-column parameters), not
-// by bytes in flight - with the ring they were no faster (RMSNorm) or slower (LayerNorm: fewer resident warps).
+// walk rows the same way but keep only the next row in flight, in registers: see row_load.
 constexpr int kRing = 4;
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
@@ -100,6 +82,50 @@ static int persistent_grid(int threads, size_t smem, int rows) {
   return static_cast<int>(rows < cap ? rows : cap);
 }
 
+// ------------------------------------------------------------ row kernels with the next row in registers
+// RMSNorm rows: persistent CTAs of 128 threads, a thread's 16-byte vectors of the next row (raw bf16, NV x 4
+// registers) are requested before the arithmetic on the present one, so that loads are in flight all the time.  With one
+// row per short-lived CTA a row spent most of its 4 us waiting - for its own load, for the CTA's launch - and seven
+// resident CTAs per SM did not cover that.  L1 is left to the per-column weights (20 KB for 5120 columns).  (LayerNorm with
+// modulation, three reductions and twice the parameters, gains nothing from this: it is bound by instruction latency.)
+template <int NV>
+__device__ __forceinline__ void row_load(uint4 (&raw)[NV], const __nv_bfloat16* row, int nvec) {
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int vi = threadIdx.x + i * kRowThreads;
+    if (vi < nvec)
+      asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(raw[i].x), "=r"(raw[i].y), "=r"(raw[i].z), "=r"(raw[i].w)
+                   : "l"(row + vi * 8));
+  }
+}
+// Sums / maxima over the CTA's four warps, R at once with one barrier.  `red` must be another buffer than the previous
+// reduction's: a thread that writes it again has passed a barrier which every reader reached after its read.
+template <int R>
+__device__ __forceinline__ void row_sum(float (&v)[R], float (&red)[4][R]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = warp_sum(v[r]);
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) red[threadIdx.x >> 5][r] = v[r];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = red[0][r] + red[1][r] + red[2][r] + red[3][r];
+}
+template <int R>
+__device__ __forceinline__ void row_max(float (&v)[R], float (&red)[4][R]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = warp_max(v[r]);
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) red[threadIdx.x >> 5][r] = v[r];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = fmaxf(fmaxf(red[0][r], red[1][r]), fmaxf(red[2][r], red[3][r]));
+}
+
 // ------------------------------------------------------------ ln_modulate
 // y = LayerNorm(x; eps, no affine) * (1 + scale[d]) + shift[d]
 // NV = 128-bit vectors per thread (row width D <= 128 * 8 * NV).
@@ -112,7 +138,7 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
                                                                   const float* __restrict__ scale_b, void* __restrict__ y,
                                                                   int64_t ld_y, float* __restrict__ row_scale, int M,
                                                                   int D, float eps) {
-  __shared__ float red[4];
+  __shared__ float red[3][4][1];
   const int row = blockIdx.x;
   if (row >= M) return;
   // rows below split_row take the first modulation vectors, the rest the second (text rows precede image rows
@@ -142,7 +168,9 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
       for (int j = 0; j < 4; ++j) v[i][j] = make_float2(0.f, 0.f);
     }
   }
-  const float mean = block_sum_128(s2.x + s2.y, red) / static_cast<float>(D);
+  float t[1] = {s2.x + s2.y};
+  row_sum<1>(t, red[0]);
+  const float mean = t[0] / static_cast<float>(D);
   const float2 nmean = make_float2(-mean, -mean);
   float2 q2 = make_float2(0.f, 0.f);
 #pragma unroll
@@ -156,7 +184,9 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
       }
     }
   }
-  const float var = block_sum_128(q2.x + q2.y, red) / static_cast<float>(D);
+  t[0] = q2.x + q2.y;
+  row_sum<1>(t, red[1]);
+  const float var = t[0] / static_cast<float>(D);
   const float rstd = rsqrtf(var + eps);
   const float2 rstd2 = make_float2(rstd, rstd), one2 = make_float2(1.f, 1.f);
   float amax = 0.f;
@@ -176,7 +206,7 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
       for (int j = 0; j < 4; ++j) {
         const float2 o = __ffma2_rn(__fmul2_rn(v[i][j], rstd2), __fadd2_rn(one2, sc[j]), sh[j]);
         v[i][j] = o;
-        amax = fmaxf(amax, fmaxf(fabsf(o.x), fabsf(o.y)));
+        amax = max3f(amax, fabsf(o.x), fabsf(o.y));
       }
     }
   }
@@ -193,7 +223,9 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
       }
     }
   } else {
-    amax = block_max_128(amax, red);
+    t[0] = amax;
+    row_max<1>(t, red[2]);
+    amax = t[0];
     const float qmax = (OUT == 1) ? 448.0f : 127.0f;
     const float sc = row_scale_from_amax(amax, qmax);
     const float inv = 1.0f / sc;
@@ -321,67 +353,78 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_heads_kernel(__nv_bfloat16* 
 // One CTA per row; in place.  rope == nullptr skips the rotation.
 // The output may be "chunked": column c of row m goes to out[(c / chunk_cols) * chunk_stride + m * ld_out +
 // c % chunk_cols] - the per-peer-contiguous send layout of a head/sequence all-to-all ([P][rows][D/P]).
+// Bound by HBM: 4 bytes an element and 512 bytes of factors a row.  32760 x 5120 with RoPE: 162 -> 119 us
+// (5.8 TB/s, 0.88 of the copy rate); 4608 x 3072 18.5 -> 12.4.
 template <int NV>
-__global__ void __launch_bounds__(kRowThreads) rmsnorm_full_rope_kernel(const __nv_bfloat16* buf, int64_t ld,
-                                                                        __nv_bfloat16* out, int64_t ld_out,
-                                                                        int chunk_cols, int64_t chunk_stride, int M,
-                                                                        int D, const float* __restrict__ w,
-                                                                        const float2* __restrict__ rope,
-                                                                        int rope_row0, float eps) {
-  __shared__ float red[4];
-  const int row = blockIdx.x;
-  if (row >= M) return;
+__global__ void __launch_bounds__(kRowThreads, (NV <= 3 ? 7 : NV <= 5 ? 5 : 3)) rmsnorm_full_rope_kernel(
+    const __nv_bfloat16* buf, int64_t ld, __nv_bfloat16* out, int64_t ld_out, int chunk_cols, int64_t chunk_stride, int M,
+    int D, const float* __restrict__ w, const float2* __restrict__ rope, int rope_row0, float eps) {
+  __shared__ float red[2][4][1];
   const int nvec = D >> 3;
-  const __nv_bfloat16* xr = buf + static_cast<int64_t>(row) * ld;
-  // this row's RoPE factors (512 bytes, used only after the reduction) start their trip from L2 now
-  if (rope && threadIdx.x < 4)
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(rope + (static_cast<int64_t>(rope_row0) + row) * 64 + threadIdx.x * 16));
-  // packed fp32 arithmetic (two lanes per issue slot), operations in the order of the scalar form: (x * r) * w
-  float2 v[NV][4];
-  float2 ss2 = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int vi = threadIdx.x + i * kRowThreads;
-    if (vi < nvec) {
-      bf16x8 p = *reinterpret_cast<const bf16x8*>(xr + vi * 8);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[i][j] = unpack_bf16x2(p.u[j]);
-        ss2 = __ffma2_rn(v[i][j], v[i][j], ss2);
-      }
+  // a thread's vectors are 1024 columns apart, a multiple of the head width: the same four (cos, sin) pairs serve them all
+  const float4* rope_mine = reinterpret_cast<const float4*>(rope + ((threadIdx.x * 8) & 127) / 2);
+  uint4 raw[NV];
+  float4 rot[2] = {make_float4(1.f, 0.f, 1.f, 0.f), make_float4(1.f, 0.f, 1.f, 0.f)};
+  auto load = [&](int r) {
+    row_load<NV>(raw, buf + static_cast<int64_t>(r) * ld, nvec);
+    if (rope) {
+      rot[0] = __ldg(rope_mine + (static_cast<int64_t>(rope_row0) + r) * 32);
+      rot[1] = __ldg(rope_mine + (static_cast<int64_t>(rope_row0) + r) * 32 + 1);
     }
-  }
-  const float r = rsqrtf(block_sum_128(ss2.x + ss2.y, red) / static_cast<float>(D) + eps);
-  const float2 r2 = make_float2(r, r);
+  };
+  int row = blockIdx.x, it = 0;
+  if (row < M) load(row);
+  for (; row < M; row += gridDim.x, ++it) {
+    // packed fp32 arithmetic (two lanes per issue slot), operations in the order of the scalar form: (x * r) * w
+    float2 v[NV][4];
+    float2 ss2 = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int vi = threadIdx.x + i * kRowThreads;
-    if (vi < nvec) {
-      const float4 w0 = *reinterpret_cast<const float4*>(w + vi * 8);
-      const float4 w1 = *reinterpret_cast<const float4*>(w + vi * 8 + 4);
-      const float2 ww[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y),
-                            make_float2(w1.z, w1.w)};
-      float2 o[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) o[j] = __fmul2_rn(__fmul2_rn(v[i][j], r2), ww[j]);
-      if (rope) {
-        const int pair0 = ((vi * 8) & 127) >> 1;  // pair index inside the head
-        const float2* rr = rope + (static_cast<int64_t>(rope_row0) + row) * 64 + pair0;
+    for (int i = 0; i < NV; ++i) {
+      if (threadIdx.x + i * kRowThreads < nvec) {
+        const uint32_t u[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float2 c = rr[j];
-          const float a = o[j].x, b = o[j].y;
-          o[j].x = c.x * a - c.y * b;
-          o[j].y = c.y * a + c.x * b;
+          v[i][j] = unpack_bf16x2(u[j]);
+          ss2 = __ffma2_rn(v[i][j], v[i][j], ss2);
         }
       }
-      bf16x8 p;
+    }
+    const float2 cs[4] = {make_float2(rot[0].x, rot[0].y), make_float2(rot[0].z, rot[0].w), make_float2(rot[1].x, rot[1].y),
+                          make_float2(rot[1].z, rot[1].w)};
+    // (the next row is another row than this CTA writes: in place is fine)
+    const int next = row + static_cast<int>(gridDim.x);
+    if (next < M) load(next);
+    float ss[1] = {ss2.x + ss2.y};
+    row_sum<1>(ss, red[it & 1]);
+    const float r = rsqrtf(ss[0] / static_cast<float>(D) + eps);
+    const float2 r2 = make_float2(r, r);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) p.u[j] = pack_bf16x2(o[j].x, o[j].y);
-      const int col = vi * 8;
-      const int ck = col / chunk_cols;
-      *reinterpret_cast<bf16x8*>(out + ck * chunk_stride + static_cast<int64_t>(row) * ld_out + (col - ck * chunk_cols)) =
-          p;
+    for (int i = 0; i < NV; ++i) {
+      const int vi = threadIdx.x + i * kRowThreads;
+      if (vi < nvec) {
+        const float4 w0 = *reinterpret_cast<const float4*>(w + vi * 8);
+        const float4 w1 = *reinterpret_cast<const float4*>(w + vi * 8 + 4);
+        const float2 ww[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y),
+                              make_float2(w1.z, w1.w)};
+        float2 o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = __fmul2_rn(__fmul2_rn(v[i][j], r2), ww[j]);
+        if (rope) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float a = o[j].x, b = o[j].y;
+            o[j].x = cs[j].x * a - cs[j].y * b;
+            o[j].y = cs[j].y * a + cs[j].x * b;
+          }
+        }
+        bf16x8 p;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p.u[j] = pack_bf16x2(o[j].x, o[j].y);
+        const int col = vi * 8;
+        const int ck = chunk_cols >= D ? 0 : col / chunk_cols;
+        *reinterpret_cast<bf16x8*>(out + ck * chunk_stride + static_cast<int64_t>(row) * ld_out + (col - ck * chunk_cols)) =
+            p;
+      }
     }
   }
 }
@@ -1121,10 +1164,13 @@ int dsb_rmsnorm_full(const void* x, int64_t ld_x, void* out, int64_t ld_out, int
   const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(x);
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
   const float2* rp = reinterpret_cast<const float2*>(rope);
+  int grid = 0;
 #define DSB_RMS_CASE(NV)                                                                                          \
   case NV:                                                                                                        \
-    rmsnorm_full_rope_kernel<NV><<<M, kRowThreads, 0, st>>>(b, ld_x, o, ld_out, out_chunk_cols, out_chunk_stride, \
-                                                           M, D, w, rp, rope_row0, eps);                        \
+    grid = persistent_grid<rmsnorm_full_rope_kernel<NV>>(kRowThreads, 0, M);                                       \
+    if (grid <= 0) return DSB_ERR_CUDA;                                                                            \
+    rmsnorm_full_rope_kernel<NV><<<grid, kRowThreads, 0, st>>>(b, ld_x, o, ld_out, out_chunk_cols, out_chunk_stride, \
+                                                               M, D, w, rp, rope_row0, eps);                       \
     break;
   switch (nv) {
     DSB_RMS_CASE(1) DSB_RMS_CASE(2) DSB_RMS_CASE(3) DSB_RMS_CASE(4) DSB_RMS_CASE(5) DSB_RMS_CASE(6) DSB_RMS_CASE(7)
