@@ -901,8 +901,11 @@ __global__ void __launch_bounds__(256) dequant_gguf_kernel(const uint8_t* __rest
 
 // ------------------------------------------------------------------- gemv
 // y[n] = (sum_k W[n,k] * f(x[k])) * w_scale[n or 0] + bias[n].  The activation vector is staged once per CTA
-// in shared memory; each warp walks groups of four consecutive rows so that every 64-byte read of the
-// activations serves four weight rows and four 16-byte weight loads per lane are in flight.
+// in shared memory; each warp walks groups of R consecutive rows so that every 64-byte read of the activations serves
+// R weight rows, with U x R 16-byte weight loads per lane in flight.  The first of them are requested before the
+// activations are staged, and those come as independent 16-byte loads (a loop of one load and one SiLU per turn was most
+// of a small Linear's time): 18432 x 3072 e4m3 16.6 -> 14.6 us with the launch, 30720 x 5120 40.6 -> 35.1, 3072 x 3072
+// 11.1 -> 9.7; 400000 x 3072 runs at 6.5 TB/s.
 // WFMT: 0 bf16, 1 e4m3, 2 int8.  act_in: DSB_ACT_NONE or DSB_ACT_SILU on x; act_out: any DSB_ACT_* on y.
 template <int WFMT>
 __device__ __forceinline__ void dequant16(const uint4& p, float (&w)[16]) {
@@ -925,54 +928,91 @@ __device__ __forceinline__ void dequant16(const uint4& p, float (&w)[16]) {
   }
 }
 
-template <int WFMT>
+template <int WFMT, int R, int U>
 __global__ void __launch_bounds__(256) gemv_kernel(const void* __restrict__ W, int64_t ld_w_bytes,
                                                    const float* __restrict__ x, const float* __restrict__ w_scale,
                                                    int w_scale_stride, const float* __restrict__ bias,
                                                    float* __restrict__ y, int N, int K, int act_in, int act_out,
                                                    int accumulate) {
   extern __shared__ float xs[];
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
-    float t = x[k];
-    xs[k] = act_in == DSB_ACT_SILU ? silu(t) : t;
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
-  constexpr int R = 4;
   constexpr int EPL = (WFMT == 0) ? 8 : 16;  // elements per 16-byte load
+  constexpr int kStep = 32 * EPL;
   const int groups = (N + R - 1) / R;
-  for (int g = blockIdx.x * warps + (threadIdx.x >> 5); g < groups; g += gridDim.x * warps) {
-    const int n0 = g * R;
-    const uint8_t* wr[R];
+  uint4 p[U][R];
+  auto load = [&](int g, int k0) {
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-      wr[r] = reinterpret_cast<const uint8_t*>(W) + static_cast<int64_t>(min(n0 + r, N - 1)) * ld_w_bytes;
-    float acc[R] = {0.f, 0.f, 0.f, 0.f};
-    for (int k = lane * EPL; k < K; k += 32 * EPL) {
-      uint4 p[R];
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * kStep;
+      if (k < K) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) p[r] = *reinterpret_cast<const uint4*>(wr[r] + k * (WFMT == 0 ? 2 : 1));
-      float xv[EPL];
-#pragma unroll
-      for (int e = 0; e < EPL; e += 4) {
-        const float4 t = *reinterpret_cast<const float4*>(xs + k + e);
-        xv[e] = t.x, xv[e + 1] = t.y, xv[e + 2] = t.z, xv[e + 3] = t.w;
+        for (int r = 0; r < R; ++r)
+          asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(p[u][r].x), "=r"(p[u][r].y), "=r"(p[u][r].z), "=r"(p[u][r].w)
+                       : "l"(reinterpret_cast<const uint8_t*>(W) + static_cast<int64_t>(min(g * R + r, N - 1)) * ld_w_bytes +
+                             k * (WFMT == 0 ? 2 : 1)));
       }
+    }
+  };
+  int g = blockIdx.x * warps + (threadIdx.x >> 5);
+  if (g < groups) load(g, lane * EPL);
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {  // K is a multiple of 8
+    for (int k0 = threadIdx.x * 4; k0 < K; k0 += 4 * 1024) {
+      float4 t[4];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if constexpr (WFMT == 0) {
-          const uint32_t u[4] = {p[r].x, p[r].y, p[r].z, p[r].w};
+      for (int i = 0; i < 4; ++i)
+        if (k0 + i * 1024 < K)
+          asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(t[i].x), "=f"(t[i].y), "=f"(t[i].z), "=f"(t[i].w)
+                       : "l"(x + k0 + i * 1024));
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 f = unpack_bf16x2(u[j]);
-            acc[r] += f.x * xv[2 * j] + f.y * xv[2 * j + 1];
+      for (int i = 0; i < 4; ++i) {
+        if (k0 + i * 1024 >= K) break;
+        if (act_in == DSB_ACT_SILU) t[i] = make_float4(silu(t[i].x), silu(t[i].y), silu(t[i].z), silu(t[i].w));
+        *reinterpret_cast<float4*>(xs + k0 + i * 1024) = t[i];
+      }
+    }
+  } else {
+    for (int k = threadIdx.x; k < K; k += blockDim.x) {
+      const float t = x[k];
+      xs[k] = act_in == DSB_ACT_SILU ? silu(t) : t;
+    }
+  }
+  __syncthreads();
+  for (bool loaded = true; g < groups; g += gridDim.x * warps, loaded = false) {
+    const int n0 = g * R;
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.f;
+    for (int k0 = lane * EPL; k0 < K; k0 += U * kStep) {
+      if (!loaded) load(g, k0);
+      loaded = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + u * kStep;
+        if (k >= K) break;
+        float xv[EPL];
+#pragma unroll
+        for (int e = 0; e < EPL; e += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(xs + k + e);
+          xv[e] = t.x, xv[e + 1] = t.y, xv[e + 2] = t.z, xv[e + 3] = t.w;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if constexpr (WFMT == 0) {
+            const uint32_t q[4] = {p[u][r].x, p[u][r].y, p[u][r].z, p[u][r].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = unpack_bf16x2(q[j]);
+              acc[r] += f.x * xv[2 * j] + f.y * xv[2 * j + 1];
+            }
+          } else {
+            float w[16];
+            dequant16<WFMT>(p[u][r], w);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) acc[r] += w[e] * xv[e];
           }
-        } else {
-          float w[16];
-          dequant16<WFMT>(p[r], w);
-#pragma unroll
-          for (int e = 0; e < 16; ++e) acc[r] += w[e] * xv[e];
         }
       }
     }
@@ -981,9 +1021,9 @@ __global__ void __launch_bounds__(256) gemv_kernel(const void* __restrict__ W, i
     if (lane < R && n0 + lane < N) {
       const int n = n0 + lane;
       float a = acc[0];
-      if (lane == 1) a = acc[1];
-      if (lane == 2) a = acc[2];
-      if (lane == 3) a = acc[3];
+#pragma unroll
+      for (int r = 1; r < R; ++r)
+        if (lane == r) a = acc[r];
       const float sc = w_scale ? w_scale[static_cast<int64_t>(n) * w_scale_stride] : 1.0f;
       float o = a * sc + (bias ? bias[n] : 0.f);
       if (act_out == DSB_ACT_SILU) o = silu(o);
@@ -1340,22 +1380,35 @@ int dsb_gemv(const void* W, int64_t ld_w, int w_fmt, const float* x, const float
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const size_t smem = static_cast<size_t>(K) * 4;
   const int64_t ldb = ld_w * esz;
-  int blocks = (N + 31) / 32;  // one warp per group of four rows
-#define DSB_GEMV(F)                                                                                             \
-  {                                                                                                             \
-    auto kern = gemv_kernel<F>;                                                                                 \
-    DSB_ENSURE_SMEM(kern, 96 * 1024);                                                                           \
-    int occ = 1;                                                                                                \
+  // Rows per warp: one when the rows are long (4 KB: eight 16-byte loads a lane) and every one of them can have a warp of
+  // its own on the device at once, else four.  3072 x 3072 bf16 14.1 us with four, 10.0 with one; shorter rows lose to the
+  // extra CTAs' staging of the activations (3072 x 768 e4m3 5.4 us with four, 6.3 with one).
+#define DSB_GEMV_R(F, R, U, WHEN)                                                                                \
+  if (!done && (WHEN)) {                                                                                         \
+    auto kern = gemv_kernel<F, R, U>;                                                                            \
+    DSB_ENSURE_SMEM(kern, 96 * 1024);                                                                            \
+    int occ = 1;                                                                                                 \
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, smem) != cudaSuccess || occ < 1) occ = 1; \
-    if (blocks > occ * sm_count()) blocks = occ * sm_count(); /* exactly the resident set: no second wave */     \
-    gemv_kernel<F><<<blocks, 256, smem, st>>>(W, ldb, x, w_scale, w_scale_stride, bias, y, N, K, act_in, act_out, \
-                                               accumulate);                                                       \
+    const int resident = occ * sm_count();                                                                       \
+    const int blocks = (N + 8 * R - 1) / (8 * R);                                                                \
+    if (R == 4 || blocks <= resident) {                                                                          \
+      kern<<<blocks < resident ? blocks : resident, 256, smem, st>>>(W, ldb, x, w_scale, w_scale_stride, bias, y, N, K, \
+                                                                     act_in, act_out, accumulate);               \
+      done = true;                                                                                               \
+    }                                                                                                            \
+  }
+#define DSB_GEMV(F)                                            \
+  {                                                            \
+    bool done = false;                                         \
+    DSB_GEMV_R(F, 1, 6, static_cast<int64_t>(K) * esz >= 4096) \
+    DSB_GEMV_R(F, 4, 1, true)                                  \
   }
   if (w_fmt == DSB_FMT_BF16) DSB_GEMV(0)
   else if (w_fmt == DSB_FMT_E4M3) DSB_GEMV(1)
   else if (w_fmt == DSB_FMT_INT8) DSB_GEMV(2)
   else return DSB_ERR_ARG;
 #undef DSB_GEMV
+#undef DSB_GEMV_R
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }
 
