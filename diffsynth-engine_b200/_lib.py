@@ -44,6 +44,7 @@ _SIGS = {
     "dsb_dequant_gguf": [c_i, c_p, c_i64, c_i, c_i, c_p, c_i64, c_p],
     "dsb_cast_quant": [c_p, c_i64, c_p, c_i64, c_i, c_i, c_i, c_i, c_p],
     "dsb_gemv": [c_p, c_i64, c_i, c_p, c_p, c_i, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_p],
+    "dsb_gemv_rows": [c_p, c_i64, c_i, c_p, c_i64, c_i, c_p, c_i, c_p, c_p, c_i64, c_i, c_i, c_i, c_i, c_p],
     "dsb_timestep_embedding": [c_p, c_i, c_i, c_f, c_i, c_i, c_p, c_p],
     "dsb_cfg_euler_step": [c_p, c_p, c_p, c_f, c_f, c_p, c_i64, c_i, c_p],
     "dsb_euler_step": [c_p, c_p, c_p, c_p, c_f, c_p, c_i64, c_i, c_p],
@@ -54,6 +55,7 @@ _SIGS = {
     "dsb_flash_attn": [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i] + [c_i64] * 12 + [c_f, c_p, c_p],
     "dsb_flash_attn_out8": [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i] + [c_i64] * 12 + [c_f, c_p, c_p],
     "dsb_pack_quant_weight": [c_p, c_i64, c_i, c_p, c_i64, c_p, c_i, c_i, c_i, c_i, c_p, c_p],
+    "dsb_linear_rows": [c_p, c_i64, c_p, c_i64, c_i, c_i, c_i, c_i, c_p, c_i, c_p, c_i, c_p, c_i64, c_p, c_i64, c_p, c_p],
     "dsb_linear_static": [c_p, c_i64, c_p, c_i64, c_i, c_i, c_i, c_i, c_p, c_i, c_p, c_i, c_p, c_i64, c_p, c_p],
 }
 

@@ -67,18 +67,23 @@ template <int NV, int THREADS>
 __device__ __forceinline__ uint4 ring_read(const uint4* ring, int slot, int i) {
   return ring[(slot * NV + i) * THREADS + threadIdx.x];
 }
+// CTAs of a kernel that an SM holds (asked once per kernel and device: the query costs about as much as a launch)
+template <auto KERNEL>
+static int resident_ctas(int threads, size_t smem = 0) {
+  static std::atomic<int> per_sm[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  int n = per_sm[dev].load();
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, threads, smem) != cudaSuccess || n <= 0) n = 1;
+    per_sm[dev].store(n);
+  }
+  return n;
+}
 // grid of a persistent row kernel: the CTAs the device holds at once, at most one per row
 template <auto KERNEL>
 static int persistent_grid(int threads, size_t smem, int rows) {
-  static int per_sm[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  if (per_sm[dev] == 0) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, KERNEL, threads, smem) != cudaSuccess || n <= 0) n = 1;
-    per_sm[dev] = n;
-  }
-  const int64_t cap = static_cast<int64_t>(per_sm[dev]) * sm_count();
+  const int64_t cap = static_cast<int64_t>(resident_ctas<KERNEL>(threads, smem)) * sm_count();
   return static_cast<int>(rows < cap ? rows : cap);
 }
 
@@ -930,11 +935,14 @@ __device__ __forceinline__ void dequant16(const uint4& p, float (&w)[16]) {
 
 template <int WFMT, int R, int U>
 __global__ void __launch_bounds__(256) gemv_kernel(const void* __restrict__ W, int64_t ld_w_bytes,
-                                                   const float* __restrict__ x, const float* __restrict__ w_scale,
-                                                   int w_scale_stride, const float* __restrict__ bias,
-                                                   float* __restrict__ y, int N, int K, int act_in, int act_out,
-                                                   int accumulate) {
+                                                   const void* __restrict__ x_rows, int64_t ld_x, int x_bf16,
+                                                   const float* __restrict__ w_scale, int w_scale_stride,
+                                                   const float* __restrict__ bias, void* __restrict__ y_rows, int64_t ld_y,
+                                                   int y_bf16, int N, int K, int act_in, int act_out, int accumulate) {
   extern __shared__ float xs[];
+  // one activation row per blockIdx.y, fp32 or bf16 in and out; the arithmetic is fp32 either way
+  const float* x = reinterpret_cast<const float*>(x_rows) + blockIdx.y * ld_x;
+  const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x_rows) + blockIdx.y * ld_x;
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   constexpr int EPL = (WFMT == 0) ? 8 : 16;  // elements per 16-byte load
@@ -957,7 +965,25 @@ __global__ void __launch_bounds__(256) gemv_kernel(const void* __restrict__ W, i
   };
   int g = blockIdx.x * warps + (threadIdx.x >> 5);
   if (g < groups) load(g, lane * EPL);
-  if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {  // K is a multiple of 8
+  if (x_bf16) {
+    const bool vec = (reinterpret_cast<uintptr_t>(xb) & 15u) == 0;
+    for (int k = threadIdx.x * 8; k < K; k += 8 * 256) {  // K is a multiple of 8
+      uint4 q;
+      if (vec) {
+        q = *reinterpret_cast<const uint4*>(xb + k);
+      } else {
+        const uint16_t* h = reinterpret_cast<const uint16_t*>(xb + k);
+        q = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+      }
+      const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 t = unpack_bf16x2(u[j]);
+        if (act_in == DSB_ACT_SILU) t = make_float2(silu(t.x), silu(t.y));
+        *reinterpret_cast<float2*>(xs + k + 2 * j) = t;
+      }
+    }
+  } else if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
     for (int k0 = threadIdx.x * 4; k0 < K; k0 += 4 * 1024) {
       float4 t[4];
 #pragma unroll
@@ -1029,7 +1055,12 @@ __global__ void __launch_bounds__(256) gemv_kernel(const void* __restrict__ W, i
       if (act_out == DSB_ACT_SILU) o = silu(o);
       if (act_out == DSB_ACT_GELU_TANH) o = gelu_tanh(o);
       if (act_out == DSB_ACT_GELU) o = gelu_erf(o);
-      y[n] = accumulate ? y[n] + o : o;
+      if (y_bf16) {
+        reinterpret_cast<__nv_bfloat16*>(y_rows)[blockIdx.y * ld_y + n] = __float2bfloat16_rn(o);
+      } else {
+        float* y = reinterpret_cast<float*>(y_rows) + blockIdx.y * ld_y + n;
+        *y = accumulate ? *y + o : o;
+      }
     }
   }
 }
@@ -1208,7 +1239,6 @@ int dsb_rmsnorm_full(const void* x, int64_t ld_x, void* out, int64_t ld_out, int
 #define DSB_RMS_CASE(NV)                                                                                          \
   case NV:                                                                                                        \
     grid = persistent_grid<rmsnorm_full_rope_kernel<NV>>(kRowThreads, 0, M);                                       \
-    if (grid <= 0) return DSB_ERR_CUDA;                                                                            \
     rmsnorm_full_rope_kernel<NV><<<grid, kRowThreads, 0, st>>>(b, ld_x, o, ld_out, out_chunk_cols, out_chunk_stride, \
                                                                M, D, w, rp, rope_row0, eps);                       \
     break;
@@ -1222,6 +1252,9 @@ int dsb_rmsnorm_full(const void* x, int64_t ld_x, void* out, int64_t ld_out, int
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }
 
+static int run_gemv(const void* W, int64_t ld_w, int w_fmt, const void* x, int64_t ld_x, int x_bf16, const float* w_scale,
+                    int w_scale_stride, const float* bias, void* y, int64_t ld_y, int y_bf16, int M, int N, int K, int act_in,
+                    int act_out, int accumulate, void* stream);
 static int quant_rows_impl(const void* x, int64_t ld_x, int chunk_cols, int64_t chunk_stride, void* y, int64_t ld_y,
                            float* row_scale, int M, int K, int out_fmt, void* stream);
 
@@ -1371,6 +1404,20 @@ int dsb_cast_quant(const void* x, int64_t ld_x, void* y, int64_t ld_y, int M, in
 
 int dsb_gemv(const void* W, int64_t ld_w, int w_fmt, const float* x, const float* w_scale, int w_scale_stride,
              const float* bias, float* y, int N, int K, int act_in, int act_out, int accumulate, void* stream) {
+  return run_gemv(W, ld_w, w_fmt, x, 0, 0, w_scale, w_scale_stride, bias, y, 0, 0, 1, N, K, act_in, act_out, accumulate, stream);
+}
+
+int dsb_gemv_rows(const void* W, int64_t ld_w, int w_fmt, const void* x, int64_t ld_x, int x_bf16, const float* w_scale,
+                  int w_scale_stride, const float* bias, void* y, int64_t ld_y, int y_bf16, int M, int N, int K, void* stream) {
+  if (M < 0 || M > 65535) return DSB_ERR_ARG;
+  if (M == 0) return DSB_OK;
+  return run_gemv(W, ld_w, w_fmt, x, ld_x, x_bf16 ? 1 : 0, w_scale, w_scale_stride, bias, y, ld_y, y_bf16 ? 1 : 0, M, N, K,
+                  DSB_ACT_NONE, DSB_ACT_NONE, 0, stream);
+}
+
+static int run_gemv(const void* W, int64_t ld_w, int w_fmt, const void* x, int64_t ld_x, int x_bf16, const float* w_scale,
+                    int w_scale_stride, const float* bias, void* y, int64_t ld_y, int y_bf16, int M, int N, int K, int act_in,
+                    int act_out, int accumulate, void* stream) {
   if (!W || !x || !y || N < 0 || K <= 0 || !aligned16(W)) return DSB_ERR_ARG;
   const int esz = (w_fmt == DSB_FMT_BF16) ? 2 : 1;
   const int kq = (w_fmt == DSB_FMT_BF16) ? 8 : 16;
@@ -1387,13 +1434,14 @@ int dsb_gemv(const void* W, int64_t ld_w, int w_fmt, const float* x, const float
   if (!done && (WHEN)) {                                                                                         \
     auto kern = gemv_kernel<F, R, U>;                                                                            \
     DSB_ENSURE_SMEM(kern, 96 * 1024);                                                                            \
-    int occ = 1;                                                                                                 \
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 256, smem) != cudaSuccess || occ < 1) occ = 1; \
-    const int resident = occ * sm_count();                                                                       \
+    /* CTAs that fit: what the registers allow, and what the activations leave of 227 KB (1 KB each is reserved) */ \
+    const int occ = resident_ctas<gemv_kernel<F, R, U>>(256);                                                    \
+    const int fit = static_cast<int>((size_t(227) << 10) / (smem + 1024));                                       \
+    const int resident = (occ < fit ? occ : fit) * sm_count();                                                   \
     const int blocks = (N + 8 * R - 1) / (8 * R);                                                                \
     if (R == 4 || blocks <= resident) {                                                                          \
-      kern<<<blocks < resident ? blocks : resident, 256, smem, st>>>(W, ldb, x, w_scale, w_scale_stride, bias, y, N, K, \
-                                                                     act_in, act_out, accumulate);               \
+      kern<<<dim3(blocks < resident ? blocks : resident, M), 256, smem, st>>>(                                   \
+          W, ldb, x, ld_x, x_bf16, w_scale, w_scale_stride, bias, y, ld_y, y_bf16, N, K, act_in, act_out, accumulate); \
       done = true;                                                                                               \
     }                                                                                                            \
   }

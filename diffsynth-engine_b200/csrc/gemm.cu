@@ -837,3 +837,18 @@ extern "C" int dsb_gemm_qkv(const void* A, int64_t lda, const void* W, int64_t l
   a.nq_w = nq_w, a.nk_w = nk_w, a.d_model = d_model, a.rope = rope, a.rope_row0 = rope_row0, a.norm_eps = norm_eps;
   return dsb_gemm_group(&a, 1, fmt, status, stream);
 }
+
+extern "C" int dsb_linear_rows(const void* x, int64_t ld_x, const void* Wq, int64_t ld_w, int w_fmt, int M, int N, int K,
+                               const float* w_scale, int w_scale_stride, const float* bias, int act, void* work,
+                               int64_t work_bytes, void* out, int64_t ld_out, int* status, void* stream) {
+  if (w_fmt != DSB_FMT_E4M3 && w_fmt != DSB_FMT_INT8) return DSB_ERR_ARG;
+  if (M < 0 || N < 0 || K <= 0 || (K & 15) || !w_scale || !work || (reinterpret_cast<uintptr_t>(work) & 15u)) return DSB_ERR_ARG;
+  const int64_t rows_bytes = static_cast<int64_t>(M) * K;  // a multiple of 16: the row scales behind it are aligned
+  if (work_bytes < rows_bytes + static_cast<int64_t>(M) * 4) return DSB_ERR_ARG;
+  if (M == 0 || N == 0) return DSB_OK;
+  float* row_scale = reinterpret_cast<float*>(static_cast<unsigned char*>(work) + rows_bytes);
+  const int rc = dsb_quant_rows(x, ld_x, work, K, row_scale, M, K, w_fmt, stream);
+  if (rc != DSB_OK) return rc;
+  return dsb_gemm(work, K, Wq, ld_w, w_fmt, M, N, K, row_scale, w_scale, w_scale_stride, bias, act, 0, nullptr, nullptr, 0,
+                  out, ld_out, nullptr, 0, N, status, stream);
+}

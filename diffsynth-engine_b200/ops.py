@@ -13,11 +13,14 @@ _status = {}
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    """Device address for an argument that the binding declares as ``void*`` (None = NULL)."""
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Handle of the current stream of the current device.  Asked of the C layer directly: building the Python stream
+    object that ``torch.cuda.current_stream`` returns takes longer than a small kernel."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _require_cuda(*ts):
@@ -30,9 +33,9 @@ def _require_cuda(*ts):
         if not t.is_cuda:
             raise _lib.DsbError("dsb ops take CUDA tensors only (no CPU fallback exists)")
         if cur is None:
-            cur = torch.cuda.current_device()
-        if t.device.index != cur:
-            raise _lib.DsbError(f"tensor on cuda:{t.device.index} but the current device is cuda:{cur}: wrap the call "
+            cur = torch._C._cuda_getDevice()
+        if t.get_device() != cur:
+            raise _lib.DsbError(f"tensor on cuda:{t.get_device()} but the current device is cuda:{cur}: wrap the call "
                                 "in torch.cuda.device(tensor.device)")
 
 
@@ -43,10 +46,13 @@ def _require_bf16(t, what):
 
 def status_word(device) -> torch.Tensor:
     """Per-device int32 the kernels set to DSB_ERR_TIMEOUT when a bounded wait runs out."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
-    return _status[key]
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index
+    if key is None:
+        key = torch.cuda.current_device()
+    word = _status.get(key)
+    if word is None:
+        word = _status[key] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
+    return word
 
 
 def check_status(device=None):
@@ -278,6 +284,30 @@ def gemv(W, x, w_scale=None, bias=None, act_in=ACT_NONE, act_out=ACT_NONE, out=N
     rc = _lib.lib().dsb_gemv(_ptr(W), ld_w, _fmt_of(W), _ptr(x), _ptr(w_scale), stride, _ptr(bias), _ptr(out), N, K,
                              act_in, act_out, 1 if accumulate else 0, _stream())
     check(rc, "dsb_gemv")
+    return out
+
+
+def gemv_rows(W, x, w_scale=None, bias=None, out=None):
+    """y = (W @ x) * w_scale + bias for a few rows ``x[M, K]`` in one launch, fp32 arithmetic; ``x`` and ``out`` (default:
+    the dtype of ``x``) are float32 or bfloat16."""
+    _require_cuda(W, x, w_scale, bias, out)
+    N, K, ld_w = _rows(W)
+    M, Kx, ld_x = _rows(x)
+    if out is None:
+        out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    Mo, No, ld_y = _rows(out)
+    if Kx != K or Mo != M or No != N:
+        raise _lib.DsbError("gemv_rows operands disagree in M, N or K")
+    for t in (x, out):
+        if t.dtype != torch.bfloat16 and t.dtype != torch.float32:
+            raise _lib.DsbError(f"gemv_rows takes float32 or bfloat16 rows, got {t.dtype}")
+    for name, t, n in (("w_scale", w_scale, 1 if (w_scale is not None and w_scale.numel() == 1) else N), ("bias", bias, N)):
+        if t is not None and (t.dtype != torch.float32 or t.numel() < n or not t.is_contiguous()):
+            raise _lib.DsbError(f"gemv_rows {name} must be contiguous float32 with at least {n} elements")
+    stride = 0 if (w_scale is None or w_scale.numel() == 1) else 1
+    rc = _lib.lib().dsb_gemv_rows(_ptr(W), ld_w, _fmt_of(W), _ptr(x), ld_x, x.dtype == torch.bfloat16, _ptr(w_scale), stride,
+                                  _ptr(bias), _ptr(out), ld_y, out.dtype == torch.bfloat16, M, N, K, _stream())
+    check(rc, "dsb_gemv_rows")
     return out
 
 
@@ -571,6 +601,26 @@ def pack_quant_weight(W, fmt=FMT_E4M3, per_channel=False):
                                           _ptr(scales), N, K, fmt, 1 if per_channel else 0, _ptr(work), _stream())
     check(rc, "dsb_pack_quant_weight")
     return payload, scales
+
+
+def linear_rows(x, w, scale, bias=None, act=ACT_NONE, out=None):
+    """``dsb_linear_rows``: bf16 rows ``x[M, K]`` quantised and multiplied by the prepacked 8-bit ``w[N, K]``, two launches
+    from one call; the quantised rows and their scales live in one scratch tensor for its duration."""
+    _require_cuda(x, w, scale, bias, out)
+    _require_bf16(x, "linear_rows")
+    M, K, ld_x = _rows(x)
+    N, Kw, ld_w = _rows(w)
+    if K != Kw:
+        raise _lib.DsbError("linear_rows operands disagree in K")
+    if out is None:
+        out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    _check_gemm_io(M, N, out, None, None, col_scale=scale, bias=bias)
+    work = torch.empty(M * (K + 4), dtype=torch.uint8, device=x.device)
+    rc = _lib.lib().dsb_linear_rows(_ptr(x), ld_x, _ptr(w), ld_w, _fmt_of(w), M, N, K, _ptr(scale),
+                                    0 if scale.numel() == 1 else 1, _ptr(bias), act, _ptr(work), work.numel(), _ptr(out),
+                                    out.stride(0), _ptr(status_word(x.device)), _stream())
+    check(rc, "dsb_linear_rows")
+    return out
 
 
 def linear_static(x, w_payload, w_scale, bias=None, act=ACT_NONE, out=None):

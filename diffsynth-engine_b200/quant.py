@@ -121,33 +121,30 @@ def b200_linear(input: torch.Tensor, weight: torch.Tensor, bias=None, _origin=F.
     if not input.is_cuda:
         raise ops._lib.DsbError("b200_linear got a CPU tensor: there is no CPU fallback")
     N, K = weight.shape
-    lead = input.shape[:-1]
-    x = input.reshape(-1, K)
+    x = input if input.dim() == 2 else input.reshape(-1, K)
     M = x.shape[0]
     b32 = weight.bias_f32(bias)
-    payload = weight.data
     ext = getattr(weight, "lora_ext", None)
-    if ext is not None:
-        from .lora import linear_lora
+    if ext is None and M <= 4:
+        # conditioning vectors: bandwidth-bound GEMV on fp32 activations, weights dequantised on the fly
+        xf = x if x.dtype in (torch.bfloat16, torch.float32) else x.float()
+        if xf.stride(-1) != 1:
+            xf = xf.contiguous()
+        y = ops.gemv_rows(weight, xf, weight.scale, b32)
+    else:
         xb = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
         if xb.stride(-1) != 1 or (xb.stride(0) % 8) or (xb.data_ptr() % 16):
             xb = xb.contiguous()
-        return linear_lora(xb, payload, weight.scale, b32, ext).to(input.dtype).reshape(*lead, N)
-    if M <= 4:  # conditioning vectors: bandwidth-bound GEMV on fp32 activations, weights dequantised on the fly
-        xf = x.float().contiguous()
-        rows = [ops.gemv(payload, xf[i], weight.scale, b32) for i in range(M)]
-        y = torch.stack(rows) if M > 1 else rows[0][None]
-        return y.to(input.dtype).reshape(*lead, N)
-    xb = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
-    if xb.stride(-1) != 1 or (xb.stride(0) % 8) or (xb.data_ptr() % 16):
-        xb = xb.contiguous()
-    afmt = act_format(weight.fmt)
-    if afmt == ops.FMT_BF16:
-        y = ops.gemm(xb, payload, bias=b32)
-    else:
-        xq, rs = ops.quant_rows(xb, afmt)
-        y = ops.gemm(xq, payload, row_scale=rs, col_scale=weight.scale, bias=b32)
-    return y.to(input.dtype).reshape(*lead, N)
+        if ext is not None:
+            from .lora import linear_lora
+            y = linear_lora(xb, weight.data, weight.scale, b32, ext)
+        elif act_format(weight.fmt) == ops.FMT_BF16:
+            y = ops.gemm(xb, weight, bias=b32)
+        else:
+            y = ops.linear_rows(xb, weight, weight.scale, b32)
+    if y.dtype != input.dtype:
+        y = y.to(input.dtype)
+    return y if input.dim() == 2 else y.reshape(*input.shape[:-1], N)
 
 
 @contextmanager

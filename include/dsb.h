@@ -168,6 +168,14 @@ int dsb_gemv(const void* W, int64_t ld_w, int w_fmt, const float* x, const float
              const float* bias, float* y, int N, int K, int act_in, int act_out, int accumulate, void* stream);
 
 /*
+ * The same for a few activation rows x[M, K] in one launch (act none), x and y each fp32 or bf16 (x_bf16 / y_bf16; the
+ * arithmetic is fp32): what a Linear on a conditioning vector needs between bf16 tensors without a conversion launch on
+ * either side.  Every row reads the weights again (the L2 keeps them): meant for M <= 4.
+ */
+int dsb_gemv_rows(const void* W, int64_t ld_w, int w_fmt, const void* x, int64_t ld_x, int x_bf16, const float* w_scale,
+                  int w_scale_stride, const float* bias, void* y, int64_t ld_y, int y_bf16, int M, int N, int K, void* stream);
+
+/*
  * Sinusoidal timestep embedding of n scalars t[r] * t_scale into out[n, dim] = [cos | sin] (fp32, optionally
  * rounded to bf16 values as the reference casts to the model dtype).
  *   mode 0: fp32 angles, freq_i = exp(-ln(10000) i / (dim/2))   models/basic/timestep.py:6-44 (flip_sin_to_cos,
@@ -361,6 +369,16 @@ int dsb_unpatchify(const void* tokens, int64_t ld_tok, int C, int F, int gh, int
  */
 int dsb_pack_quant_weight(const void* W, int64_t ld_w, int src_is_bf16, void* Wq, int64_t ld_q, float* scales, int N,
                           int K, int fmt, int per_channel, float* work, void* stream);
+
+/*
+ * Quantised Linear in one call: out = act((quantise_rows(x) . Wq^T) * row_scale * w_scale + bias), i.e. dsb_quant_rows
+ * followed by dsb_gemm on caller-provided scratch (`work`, 16-byte aligned, at least M*K + 4*M bytes: the 8-bit rows, then
+ * their scales).  Arguments as of dsb_linear_static below; no size limit.
+ * Replaces the patched F.linear of utils/fp8_linear.py:27-60.
+ */
+int dsb_linear_rows(const void* x, int64_t ld_x, const void* Wq, int64_t ld_w, int w_fmt, int M, int N, int K,
+                    const float* w_scale, int w_scale_stride, const float* bias, int act, void* work, int64_t work_bytes,
+                    void* out, int64_t ld_out, int* status, void* stream);
 
 /*
  * Quantised Linear that allocates nothing: out = act((quantise_rows(x) . Wq^T) * row_scale * w_scale + bias),

@@ -52,3 +52,34 @@ def test_gemv_rows(dsb, cuda_dev, N, K, fmt):
             acc = ref.float().clone()
             dsb.ops.gemv(W, x, scale, bias, act_in=act, out=acc, accumulate=True)
             assert O.rel_l2(acc.double(), 2 * ref) < 1e-5
+
+
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 130])
+@pytest.mark.parametrize("fmt", ["bf16", "fp8_tensor", "fp8_channel", "int8_channel"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+def test_patched_linear_equals_its_parts(dsb, cuda_dev, M, fmt, dtype):
+    """The patched F.linear in every dtype and on both sides of its row limit, on strided and 3-D inputs, is bit for bit the
+    conversion, quantiser, product and cast that it stands for."""
+    from diffsynth_engine_b200 import quant
+    from diffsynth_engine_b200.packed import act_format
+    ops = dsb.ops
+    torch.manual_seed(M)
+    layer = torch.nn.Linear(256, 72).to(cuda_dev, torch.bfloat16)
+    quant.enable_b200_linear(layer, fmt)
+    w, b = layer.weight, layer.bias.float()
+    base = torch.randn(2 * M, 512, device=cuda_dev).to(dtype)
+    for x in (base[:M, :256], base[::2, 256:], base[:M, 1:257], base[:M, :256].reshape(1, M, 256)):
+        with quant.b200_inference():
+            got = layer(x)
+        rows = x.reshape(-1, 256)
+        if M <= 4:
+            want = torch.stack([ops.gemv(w.data, r.float().contiguous(), w.scale, b) for r in rows])
+        else:
+            xb = rows.to(torch.bfloat16).contiguous()
+            if fmt == "bf16":
+                want = ops.gemm(xb, w.data, bias=b)
+            else:
+                q, s = ops.quant_rows(xb, act_format(fmt))
+                want = ops.gemm(q, w.data, row_scale=s, col_scale=w.scale, bias=b)
+        assert got.dtype == dtype and got.shape == (*x.shape[:-1], 72)
+        assert torch.equal(got.reshape(M, 72), want.to(dtype))
