@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     tmem_relinquish_cg2();
   }
   tc_fence_before();
+  grid_wait();
   __syncthreads();
   cluster_sync_all();  // the peer's barriers are initialised before anyone signals them
   tc_fence_after();
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           c.load(sK + st * kKBytes + kKBytes / 2, &tmap_k, b_kf + st * 8, 64, s0);
         }
       }
+      grid_release();  // a few key tiles before this CTA is done
     }
   producer_done:;
   } else if (warp == kTmaVWarp) {
@@ -659,6 +661,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
 // l = sum_p 2^(m_p - M) l_p (the m_p are integers, so the factors are exact), out = O / l.  One warp per row,
 // four columns per lane.
 __global__ void __launch_bounds__(256) attn_combine_kernel(AttnParams p, int tail_items) {
+  grid_wait();
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int rows = kPairQ;
@@ -733,20 +736,6 @@ static int make_tmap_attn(CUtensorMap* out, int (&pos)[3], const void* base, int
 
 using namespace dsb;
 
-// Launch shape of a CTA pair per two SMs; `attr` has to outlive the configuration.
-static cudaLaunchConfig_t pair_launch(cudaLaunchAttribute* attr) {
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = 2;
-  attr->val.clusterDim.y = 1;
-  attr->val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kAttnThreads, 1, 1);
-  cfg.dynamicSmemBytes = kAttnSmem;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cfg;
-}
-
 // CTA pairs the current device holds at once (a GPC with an odd SM count leaves one out); 0 on failure.  Also opts both
 // kernels into their shared memory.
 static int resident_pairs() {
@@ -759,8 +748,16 @@ static int resident_pairs() {
       cudaFuncSetAttribute(flash_attn_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem) != cudaSuccess)
     return 0;
   cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = pair_launch(&attr);
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(sm_count()) & ~1u, 1, 1);
+  cfg.blockDim = dim3(kAttnThreads, 1, 1);
+  cfg.dynamicSmemBytes = kAttnSmem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
   if (cudaOccupancyMaxActiveClusters(&n, flash_attn_kernel<false>, &cfg) != cudaSuccess || n <= 0) n = sm_count() / 2;
   cached[dev].store(n);
   return n;
@@ -875,16 +872,13 @@ static int launch_attn(const void* q, const void* const* q_parts, int n_q_parts,
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   p.n_units = p.n_full + (p.split > 1 ? tail * p.split : 0);
-  cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = pair_launch(&attr);
-  cfg.gridDim = dim3(static_cast<unsigned>(p.n_units < pairs ? p.n_units : pairs) * 2, 1, 1);
-  cfg.stream = st;
-  const cudaError_t err = p.split > 1 ? cudaLaunchKernelEx(&cfg, flash_attn_kernel<true>, qm, tk, tv, p)
-                                      : cudaLaunchKernelEx(&cfg, flash_attn_kernel<false>, qm, tk, tv, p);
+  const dim3 grid(static_cast<unsigned>(p.n_units < pairs ? p.n_units : pairs) * 2, 1, 1);
+  const cudaError_t err = launch_kernel<2>(p.split > 1 ? flash_attn_kernel<true> : flash_attn_kernel<false>, grid, kAttnThreads,
+                                           kAttnSmem, st, qm, tk, tv, p);
   if (err != cudaSuccess) return DSB_ERR_CUDA;
   if (p.split > 1) {
     const int warps = tail * kPairQ;
-    attn_combine_kernel<<<(warps + 7) / 8, 256, 0, st>>>(p, tail);
+    if (launch_kernel(attn_combine_kernel, (warps + 7) / 8, 256, 0, st, p, tail) != cudaSuccess) return DSB_ERR_CUDA;
   }
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }

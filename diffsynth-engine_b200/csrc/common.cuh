@@ -56,6 +56,15 @@ __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+// ------------------------------------------------ programmatic dependent launch
+// The library's kernels are launched so that the next one of a stream may be set up while the last CTAs of the one before
+// are still at work: each kernel waits here, before its first access to global memory, until every grid before it has
+// completed and its writes are visible.  (Returns at once in a kernel that was launched the ordinary way.)
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// ... and allows that for the next kernel when the calling CTA is about to run out of work.  Not earlier: a waiting CTA holds
+// an SM's shared memory, which a kernel of another stream (a collective) may be waiting for.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -524,6 +533,27 @@ int make_tmap_2d(CUtensorMap* out, CUtensorMapDataType dt, int elem_bytes, const
                  uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols);
 
 int sm_count();
+
+// kernel<<<grid, threads, smem, st>>>(args...) as a programmatic dependent launch, in clusters of CLUSTER CTAs.  The kernel has
+// to call grid_wait().
+template <int CLUSTER = 1, typename... P, typename... A>
+static inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CLUSTER;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = CLUSTER > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // Opt a kernel into more than 48 KiB of dynamic shared memory, once per device.
 #define DSB_ENSURE_SMEM(kernel, bytes)                                                                   \

@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
                                                                   const float* __restrict__ scale_b, void* __restrict__ y,
                                                                   int64_t ld_y, float* __restrict__ row_scale, int M,
                                                                   int D, float eps) {
+  grid_wait();
   __shared__ float red[3][4][1];
   const int row = blockIdx.x;
   if (row >= M) return;
@@ -256,6 +257,7 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
       }
     }
   }
+  grid_release();
 }
 
 template <int OUT>
@@ -266,8 +268,8 @@ static int launch_ln_modulate(const void* x, int64_t ld_x, const float* shift, c
   const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x);
 #define DSB_LN_CASE(NV)                                                                                         \
   case NV:                                                                                                      \
-    ln_modulate_kernel<NV, OUT><<<M, kRowThreads, 0, st>>>(xp, ld_x, shift, scale, split_row, shift_b, scale_b, y, ld_y, \
-                                                           row_scale, M, D, eps);                                  \
+    launch_kernel(ln_modulate_kernel<NV, OUT>, M, kRowThreads, 0, st, xp, ld_x, shift, scale, split_row, shift_b,    \
+                       scale_b, y, ld_y, row_scale, M, D, eps);                                  \
     break;
   switch (nv) {
     DSB_LN_CASE(1) DSB_LN_CASE(2) DSB_LN_CASE(3) DSB_LN_CASE(4) DSB_LN_CASE(5) DSB_LN_CASE(6) DSB_LN_CASE(7)
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const __nv_bfloat16*
                                                             const float* __restrict__ gate,
                                                             __nv_bfloat16* __restrict__ out, int64_t ld_o, int M,
                                                             int D) {
+  grid_wait();
   const int nvec = D >> 3;
   const int64_t total = static_cast<int64_t>(M) * nvec;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const __nv_bfloat16*
     }
     *reinterpret_cast<bf16x8*>(out + r * ld_o + c) = o;
   }
+  grid_release();
 }
 
 // ---------------------------------------------------- rmsnorm_rope_heads
@@ -323,6 +327,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_heads_kernel(__nv_bfloat16* 
                                                                  const float* __restrict__ w_k,
                                                                  const float2* __restrict__ rope, int rope_row0,
                                                                  float eps) {
+  grid_wait();
   const int warps_per_block = blockDim.x >> 5;
   const int64_t wid = static_cast<int64_t>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -350,6 +355,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_heads_kernel(__nv_bfloat16* 
   o.x = pack_bf16x2(x0, x1);
   o.y = pack_bf16x2(x2, x3);
   *reinterpret_cast<uint2*>(p) = o;
+  grid_release();
 }
 
 // ------------------------------------------------------ rmsnorm_full_rope
@@ -364,6 +370,7 @@ template <int NV>
 __global__ void __launch_bounds__(kRowThreads, (NV <= 3 ? 7 : NV <= 5 ? 5 : 3)) rmsnorm_full_rope_kernel(
     const __nv_bfloat16* buf, int64_t ld, __nv_bfloat16* out, int64_t ld_out, int chunk_cols, int64_t chunk_stride, int M,
     int D, const float* __restrict__ w, const float2* __restrict__ rope, int rope_row0, float eps) {
+  grid_wait();
   __shared__ float red[2][4][1];
   const int nvec = D >> 3;
   // a thread's vectors are 1024 columns apart, a multiple of the head width: the same four (cos, sin) pairs serve them all
@@ -432,6 +439,7 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 3 ? 7 : NV <= 5 ? 5 : 3)) 
       }
     }
   }
+  grid_release();
 }
 
 // ------------------------------------------------------------- quant_rows
@@ -443,6 +451,7 @@ __global__ void __launch_bounds__(256) quant_rows_ring_kernel(const __nv_bfloat1
                                                               int chunk_cols, int64_t chunk_stride,
                                                               uint8_t* __restrict__ y, int64_t ld_y,
                                                               float* __restrict__ row_scale, int M, int K) {
+  grid_wait();
   __shared__ float red[8];
   extern __shared__ uint4 ring[];
   const int nvec = K >> 3;
@@ -507,6 +516,7 @@ __global__ void __launch_bounds__(256) quant_rows_ring_kernel(const __nv_bfloat1
       }
     }
   }
+  grid_release();
 }
 
 // Wider rows: one CTA per row, the row is read twice (the second read is served by L1/L2).
@@ -515,6 +525,7 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const __nv_bfloat16* __
                                                          int chunk_cols, int64_t chunk_stride,
                                                          uint8_t* __restrict__ y, int64_t ld_y,
                                                          float* __restrict__ row_scale, int M, int K) {
+  grid_wait();
   __shared__ float red[8];
   const int row = blockIdx.x;
   if (row >= M) return;
@@ -566,6 +577,7 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const __nv_bfloat16* __
     }
     *reinterpret_cast<uint2*>(yr + vi * 8) = o;
   }
+  grid_release();
 }
 
 // ------------------------------------------------------------- patchify / unpatchify
@@ -579,6 +591,7 @@ template <int OUT>
 __global__ void __launch_bounds__(256) patchify_kernel(const __nv_bfloat16* __restrict__ lat, int C, int F, int gh, int gw,
                                                        int row0, int n_rows, void* __restrict__ out, int64_t ld_out,
                                                        float* __restrict__ row_scale) {
+  grid_wait();
   constexpr int kMaxPairs = 8;  // pairs per lane: C*2 <= 256
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -623,6 +636,7 @@ __global__ void __launch_bounds__(256) patchify_kernel(const __nv_bfloat16* __re
       }
     }
   }
+  grid_release();
 }
 
 // unpatchify: token rows [tokens, >= C*4] -> latents [C, F, 2*gh, 2*gw].  c_fastest = 1: feature (py*2 + pz)*C + c
@@ -630,6 +644,7 @@ __global__ void __launch_bounds__(256) patchify_kernel(const __nv_bfloat16* __re
 // One thread per horizontally adjacent output pair.
 __global__ void __launch_bounds__(256) unpatchify_kernel(const __nv_bfloat16* __restrict__ tok, int64_t ld_tok, int C, int F,
                                                          int gh, int gw, int c_fastest, __nv_bfloat16* __restrict__ out) {
+  grid_wait();
   const int64_t total = static_cast<int64_t>(C) * F * (2 * gh) * gw;  // pairs
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -648,6 +663,7 @@ __global__ void __launch_bounds__(256) unpatchify_kernel(const __nv_bfloat16* __
     o.y = row[f1];
     *reinterpret_cast<__nv_bfloat162*>(out + i * 2) = o;
   }
+  grid_release();
 }
 
 // ------------------------------------------------------------- cast_quant
@@ -664,6 +680,7 @@ __device__ __forceinline__ float e4m3_value(float v) {
 template <int OUT, bool SPLIT>
 __global__ void __launch_bounds__(256) cast_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ld_x,
                                                          uint8_t* __restrict__ y, int64_t ld_y, int M, int D) {
+  grid_wait();
   const int nvec = D >> 3;
   const int64_t total = static_cast<int64_t>(M) * nvec;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -698,6 +715,7 @@ __global__ void __launch_bounds__(256) cast_quant_kernel(const __nv_bfloat16* __
       *reinterpret_cast<uint2*>(dst + D) = lo;
     }
   }
+  grid_release();
 }
 
 // ---------------------------------------------------------- dequant_q8_0
@@ -939,6 +957,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(const void* __restrict__ W, i
                                                    const float* __restrict__ w_scale, int w_scale_stride,
                                                    const float* __restrict__ bias, void* __restrict__ y_rows, int64_t ld_y,
                                                    int y_bf16, int N, int K, int act_in, int act_out, int accumulate) {
+  grid_wait();
   extern __shared__ float xs[];
   // one activation row per blockIdx.y, fp32 or bf16 in and out; the arithmetic is fp32 either way
   const float* x = reinterpret_cast<const float*>(x_rows) + blockIdx.y * ld_x;
@@ -1063,6 +1082,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(const void* __restrict__ W, i
       }
     }
   }
+  grid_release();
 }
 
 // ------------------------------------------------------------ euler step
@@ -1073,6 +1093,7 @@ __global__ void __launch_bounds__(256) euler_step_kernel(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ init,
                                                          const __nv_bfloat16* __restrict__ mask, float dt,
                                                          __nv_bfloat16* __restrict__ out, int64_t n) {
+  grid_wait();
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     float m = __bfloat162float(model_out[i]);
@@ -1088,18 +1109,21 @@ __global__ void __launch_bounds__(256) euler_step_kernel(const __nv_bfloat16* __
     const float step = __bfloat162float(__float2bfloat16(m * dt));
     out[i] = __float2bfloat16(__bfloat162float(latents[i]) + step);
   }
+  grid_release();
 }
 __global__ void __launch_bounds__(256) euler_step_f32_kernel(const float* __restrict__ latents,
                                                              const float* __restrict__ model_out,
                                                              const float* __restrict__ init,
                                                              const float* __restrict__ mask, float dt,
                                                              float* __restrict__ out, int64_t n) {
+  grid_wait();
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     float m = model_out[i];
     if (mask) m = m * mask[i] + init[i] * (1.0f - mask[i]);
     out[i] = latents[i] + m * dt;
   }
+  grid_release();
 }
 
 // ------------------------------------------------------- timestep embedding
@@ -1107,6 +1131,7 @@ __global__ void __launch_bounds__(256) euler_step_f32_kernel(const float* __rest
 // mode 1: fp64 sinusoid [cos | sin], freq_i = 10000^(-i / half)               (Wan)
 __global__ void timestep_embedding_kernel(const float* __restrict__ t, int n, int dim, float t_scale, int mode,
                                           int round_bf16, float* __restrict__ out) {
+  grid_wait();
   const int half = dim / 2;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n * half) return;
@@ -1126,6 +1151,7 @@ __global__ void timestep_embedding_kernel(const float* __restrict__ t, int n, in
   }
   out[r * dim + i] = c;
   out[r * dim + half + i] = s;
+  grid_release();
 }
 
 // ------------------------------------------------- CFG combine + euler step
@@ -1135,22 +1161,26 @@ __global__ void __launch_bounds__(256) cfg_euler_step_kernel(const __nv_bfloat16
                                                              const __nv_bfloat16* __restrict__ pos,
                                                              const __nv_bfloat16* __restrict__ neg, float cfg, float dt,
                                                              __nv_bfloat16* __restrict__ out, int64_t n) {
+  grid_wait();
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float p = __bfloat162float(pos[i]), q = __bfloat162float(neg[i]);
     const float m = rbf(q + rbf(cfg * rbf(p - q)));
     out[i] = __float2bfloat16(__bfloat162float(latents[i]) + rbf(m * dt));
   }
+  grid_release();
 }
 __global__ void __launch_bounds__(256) cfg_euler_step_f32_kernel(const float* __restrict__ latents,
                                                                  const float* __restrict__ pos,
                                                                  const float* __restrict__ neg, float cfg, float dt,
                                                                  float* __restrict__ out, int64_t n) {
+  grid_wait();
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float m = neg[i] + cfg * (pos[i] - neg[i]);
     out[i] = latents[i] + m * dt;
   }
+  grid_release();
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -1201,7 +1231,7 @@ int dsb_gate_residual(const void* x, int64_t ld_x, const void* y, int64_t ld_y, 
   int blocks = static_cast<int>((total + 255) / 256);
   const int cap = sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  gate_residual_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(gate_residual_kernel, blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<const __nv_bfloat16*>(x), ld_x, reinterpret_cast<const __nv_bfloat16*>(y), ld_y, gate,
       reinterpret_cast<__nv_bfloat16*>(out), ld_o, M, D);
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
@@ -1215,7 +1245,7 @@ int dsb_rmsnorm_rope_heads(void* buf, int64_t ld, int S, int H, int head_dim, in
   if (S == 0) return DSB_OK;
   const int64_t total = static_cast<int64_t>(S) * nsel * H;
   const int blocks = static_cast<int>((total + 7) / 8);
-  rmsnorm_rope_heads_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(rmsnorm_rope_heads_kernel, blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<__nv_bfloat16*>(buf), ld, S, H, nsel, w_q, w_k ? w_k : w_q,
       reinterpret_cast<const float2*>(rope), rope_row0, eps);
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
@@ -1239,8 +1269,8 @@ int dsb_rmsnorm_full(const void* x, int64_t ld_x, void* out, int64_t ld_out, int
 #define DSB_RMS_CASE(NV)                                                                                          \
   case NV:                                                                                                        \
     grid = persistent_grid<rmsnorm_full_rope_kernel<NV>>(kRowThreads, 0, M);                                       \
-    rmsnorm_full_rope_kernel<NV><<<grid, kRowThreads, 0, st>>>(b, ld_x, o, ld_out, out_chunk_cols, out_chunk_stride, \
-                                                               M, D, w, rp, rope_row0, eps);                       \
+    launch_kernel(rmsnorm_full_rope_kernel<NV>, grid, kRowThreads, 0, st, b, ld_x, o, ld_out, out_chunk_cols,     \
+                       out_chunk_stride, M, D, w, rp, rope_row0, eps);                       \
     break;
   switch (nv) {
     DSB_RMS_CASE(1) DSB_RMS_CASE(2) DSB_RMS_CASE(3) DSB_RMS_CASE(4) DSB_RMS_CASE(5) DSB_RMS_CASE(6) DSB_RMS_CASE(7)
@@ -1288,8 +1318,7 @@ static int quant_rows_impl(const void* x, int64_t ld_x, int chunk_cols, int64_t 
     constexpr size_t smem = static_cast<size_t>(kRing) * NV * 256 * 16;                                       \
     DSB_ENSURE_SMEM((quant_rows_ring_kernel<OUT, NV>), static_cast<int>(smem));                               \
     const int grid = persistent_grid<quant_rows_ring_kernel<OUT, NV>>(256, smem, M);                          \
-    if (grid <= 0) return DSB_ERR_CUDA;                                                                       \
-    quant_rows_ring_kernel<OUT, NV><<<grid, 256, smem, st>>>(xp, ld_x, chunk_cols, chunk_stride, yp, ld_y,    \
+    launch_kernel(quant_rows_ring_kernel<OUT, NV>, grid, 256, smem, st, xp, ld_x, chunk_cols, chunk_stride, yp, ld_y,    \
                                                              row_scale, M, K);                                \
   }
 #define DSB_QR_FMT(OUT)                                                                                       \
@@ -1299,7 +1328,7 @@ static int quant_rows_impl(const void* x, int64_t ld_x, int chunk_cols, int64_t 
     case 3: DSB_QR_RING(OUT, 3) break;                                                                        \
     case 4: DSB_QR_RING(OUT, 4) break;                                                                        \
     default:                                                                                                  \
-      quant_rows_kernel<OUT><<<M, 256, 0, st>>>(xp, ld_x, chunk_cols, chunk_stride, yp, ld_y, row_scale, M, K); \
+      launch_kernel(quant_rows_kernel<OUT>, M, 256, 0, st, xp, ld_x, chunk_cols, chunk_stride, yp, ld_y, row_scale, M, K); \
   }
   if (out_fmt == DSB_FMT_E4M3) {
     DSB_QR_FMT(1)
@@ -1392,11 +1421,11 @@ int dsb_cast_quant(const void* x, int64_t ld_x, void* y, int64_t ld_y, int M, in
   const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x);
   uint8_t* yp = reinterpret_cast<uint8_t*>(y);
   if (out_fmt == DSB_FMT_E4M3 && split)
-    cast_quant_kernel<1, true><<<blocks, 256, 0, st>>>(xp, ld_x, yp, ld_y, M, D);
+    launch_kernel(cast_quant_kernel<1, true>, blocks, 256, 0, st, xp, ld_x, yp, ld_y, M, D);
   else if (out_fmt == DSB_FMT_E4M3)
-    cast_quant_kernel<1, false><<<blocks, 256, 0, st>>>(xp, ld_x, yp, ld_y, M, D);
+    launch_kernel(cast_quant_kernel<1, false>, blocks, 256, 0, st, xp, ld_x, yp, ld_y, M, D);
   else if (out_fmt == DSB_FMT_INT8)
-    cast_quant_kernel<2, false><<<blocks, 256, 0, st>>>(xp, ld_x, yp, ld_y, M, D);
+    launch_kernel(cast_quant_kernel<2, false>, blocks, 256, 0, st, xp, ld_x, yp, ld_y, M, D);
   else
     return DSB_ERR_ARG;
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
@@ -1440,8 +1469,8 @@ static int run_gemv(const void* W, int64_t ld_w, int w_fmt, const void* x, int64
     const int resident = (occ < fit ? occ : fit) * sm_count();                                                   \
     const int blocks = (N + 8 * R - 1) / (8 * R);                                                                \
     if (R == 4 || blocks <= resident) {                                                                          \
-      kern<<<dim3(blocks < resident ? blocks : resident, M), 256, smem, st>>>(                                   \
-          W, ldb, x, ld_x, x_bf16, w_scale, w_scale_stride, bias, y, ld_y, y_bf16, N, K, act_in, act_out, accumulate); \
+      launch_kernel(kern, dim3(blocks < resident ? blocks : resident, M), 256, smem, st, W, ldb, x, ld_x, x_bf16, \
+                         w_scale, w_scale_stride, bias, y, ld_y, y_bf16, N, K, act_in, act_out, accumulate);     \
       done = true;                                                                                               \
     }                                                                                                            \
   }
@@ -1464,7 +1493,7 @@ int dsb_timestep_embedding(const float* t, int n, int dim, float t_scale, int mo
                            void* stream) {
   if (!t || !out || n <= 0 || dim <= 0 || (dim & 1) || (mode != 0 && mode != 1)) return DSB_ERR_ARG;
   const int total = n * (dim / 2);
-  timestep_embedding_kernel<<<(total + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(timestep_embedding_kernel, (total + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream),
       t, n, dim, t_scale, mode, round_bf16, out);
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }
@@ -1478,12 +1507,12 @@ int dsb_cfg_euler_step(const void* latents, const void* pos, const void* neg, fl
   if (blocks > cap) blocks = cap;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (is_f32)
-    cfg_euler_step_f32_kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<const float*>(latents),
+    launch_kernel(cfg_euler_step_f32_kernel, blocks, 256, 0, st, reinterpret_cast<const float*>(latents),
                                                       reinterpret_cast<const float*>(pos),
                                                       reinterpret_cast<const float*>(neg), cfg_scale, dt,
                                                       reinterpret_cast<float*>(out), n);
   else
-    cfg_euler_step_kernel<<<blocks, 256, 0, st>>>(
+    launch_kernel(cfg_euler_step_kernel, blocks, 256, 0, st,
         reinterpret_cast<const __nv_bfloat16*>(latents), reinterpret_cast<const __nv_bfloat16*>(pos),
         reinterpret_cast<const __nv_bfloat16*>(neg), cfg_scale, dt, reinterpret_cast<__nv_bfloat16*>(out), n);
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
@@ -1499,13 +1528,13 @@ int dsb_patchify(const void* latents, int C, int F, int gh, int gw, int row0, in
   const __nv_bfloat16* lat = reinterpret_cast<const __nv_bfloat16*>(latents);
   if (out_fmt == DSB_FMT_BF16) {
     if ((reinterpret_cast<uintptr_t>(out) & 3u) || (ld_out & 1)) return DSB_ERR_ARG;
-    patchify_kernel<0><<<blocks, 256, 0, st>>>(lat, C, F, gh, gw, row0, n_rows, out, ld_out, nullptr);
+    launch_kernel(patchify_kernel<0>, blocks, 256, 0, st, lat, C, F, gh, gw, row0, n_rows, out, ld_out, nullptr);
   } else if (out_fmt == DSB_FMT_E4M3 || out_fmt == DSB_FMT_INT8) {
     if (!row_scale || (reinterpret_cast<uintptr_t>(out) & 1u) || (ld_out & 1)) return DSB_ERR_ARG;
     if (out_fmt == DSB_FMT_E4M3)
-      patchify_kernel<1><<<blocks, 256, 0, st>>>(lat, C, F, gh, gw, row0, n_rows, out, ld_out, row_scale);
+      launch_kernel(patchify_kernel<1>, blocks, 256, 0, st, lat, C, F, gh, gw, row0, n_rows, out, ld_out, row_scale);
     else
-      patchify_kernel<2><<<blocks, 256, 0, st>>>(lat, C, F, gh, gw, row0, n_rows, out, ld_out, row_scale);
+      launch_kernel(patchify_kernel<2>, blocks, 256, 0, st, lat, C, F, gh, gw, row0, n_rows, out, ld_out, row_scale);
   } else {
     return DSB_ERR_ARG;
   }
@@ -1521,7 +1550,7 @@ int dsb_unpatchify(const void* tokens, int64_t ld_tok, int C, int F, int gh, int
   int blocks = static_cast<int>((total + 255) / 256);
   const int cap = sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  unpatchify_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  launch_kernel(unpatchify_kernel, blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream),
       reinterpret_cast<const __nv_bfloat16*>(tokens), ld_tok, C, F, gh, gw, c_fastest ? 1 : 0,
       reinterpret_cast<__nv_bfloat16*>(out));
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
@@ -1536,13 +1565,13 @@ int dsb_euler_step(const void* latents, const void* model_out, const void* init,
   if (blocks > cap) blocks = cap;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (is_f32)
-    euler_step_f32_kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<const float*>(latents),
+    launch_kernel(euler_step_f32_kernel, blocks, 256, 0, st, reinterpret_cast<const float*>(latents),
                                                   reinterpret_cast<const float*>(model_out),
                                                   reinterpret_cast<const float*>(init),
                                                   reinterpret_cast<const float*>(mask), dt,
                                                   reinterpret_cast<float*>(out), n);
   else
-    euler_step_kernel<<<blocks, 256, 0, st>>>(
+    launch_kernel(euler_step_kernel, blocks, 256, 0, st,
         reinterpret_cast<const __nv_bfloat16*>(latents), reinterpret_cast<const __nv_bfloat16*>(model_out),
         reinterpret_cast<const __nv_bfloat16*>(init), reinterpret_cast<const __nv_bfloat16*>(mask), dt,
         reinterpret_cast<__nv_bfloat16*>(out), n);

@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
   }
   tc_fence_before();
+  grid_wait();
   __syncthreads();
   if constexpr (CTAS == 2) cluster_sync_all();  // the peer's barriers are initialised before anyone signals them
   tc_fence_after();
@@ -227,6 +228,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
         }
       }
+      grid_release();  // one epilogue and a few K slabs before this CTA is done
     }
   producer_done:;
   } else if (warp == 1) {
@@ -593,32 +595,31 @@ static int launch_group(GemmGroup& grp, cudaStream_t st) {
   for (int i = 0; i < grp.count; ++i) tiles += grp.p[i].num_tiles;
   if constexpr (CTAS == 1) {
     const int grid = tiles < sm_count() ? tiles : sm_count();
-    kern<<<grid, kGemmThreads, SM::kTotal, st>>>(grp);
+    if (launch_kernel(kern, grid, kGemmThreads, SM::kTotal, st, grp) != cudaSuccess) return DSB_ERR_CUDA;
   } else {
     // persistent grid = the CTA pairs the device can hold at once (GPCs with an odd SM count leave one SM out)
     static int resident_pairs[64] = {0};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DSB_ERR_CUDA;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(kGemmThreads, 1, 1);
-    cfg.dynamicSmemBytes = SM::kTotal;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     if (resident_pairs[dev] == 0) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.blockDim = dim3(kGemmThreads, 1, 1);
+      cfg.dynamicSmemBytes = SM::kTotal;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
       cfg.gridDim = dim3(sm_count() & ~1, 1, 1);
       int n = 0;
       if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = sm_count() / 2;
       resident_pairs[dev] = n;
     }
     const int units = resident_pairs[dev];
-    cfg.gridDim = dim3((tiles < units ? tiles : units) * CTAS, 1, 1);
-    cfg.stream = st;
-    if (cudaLaunchKernelEx(&cfg, kern, grp) != cudaSuccess) return DSB_ERR_CUDA;
+    if (launch_kernel<2>(kern, (tiles < units ? tiles : units) * CTAS, kGemmThreads, SM::kTotal, st, grp) != cudaSuccess)
+      return DSB_ERR_CUDA;
   }
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }
