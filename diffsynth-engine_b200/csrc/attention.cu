@@ -276,143 +276,143 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   if (threadIdx.x == 0 && *tmem_slot != 0) *abort_flag = 1;
 
   if (warp < kEpiWarp0) {
-  setmaxnreg_dec<kControlRegs>();
-  if (warp == kTmaWarp) {
-    // ------------------------------------------------------------ TMA producer of Q and K
-    if (lane == 0) {
-      const uint32_t b_kf = mapa_u32(smem_u32(k_full), 0), b_qf = mapa_u32(smem_u32(q_full), 0);
-      uint32_t n = 0, t = 0;  // items and tiles so far
-      for (int u = unit0; u < p.n_units; u += n_pairs_grid, ++n) {
-        const AttnUnit w = attn_unit<SPLIT>(p, u);
-        const uint32_t qb = n & 1;
-        if (!mbar_wait(&q_empty[qb], ((n >> 1) & 1) ^ 1, abort_flag)) goto producer_done;
-        {
-          int s0 = w.q0 + static_cast<int>(rank) * kTileQ, part = 0;
-          if (p.q_rows_per_part > 0) {  // a 128-row tile never straddles two parts
-            part = min(s0 / p.q_rows_per_part, kMaxParts - 1);
-            s0 -= part * p.q_rows_per_part;
+    setmaxnreg_dec<kControlRegs>();
+    if (warp == kTmaWarp) {
+      // ------------------------------------------------------------ TMA producer of Q and K
+      if (lane == 0) {
+        const uint32_t b_kf = mapa_u32(smem_u32(k_full), 0), b_qf = mapa_u32(smem_u32(q_full), 0);
+        uint32_t n = 0, t = 0;  // items and tiles so far
+        for (int u = unit0; u < p.n_units; u += n_pairs_grid, ++n) {
+          const AttnUnit w = attn_unit<SPLIT>(p, u);
+          const uint32_t qb = n & 1;
+          if (!mbar_wait(&q_empty[qb], ((n >> 1) & 1) ^ 1, abort_flag)) goto producer_done;
+          {
+            int s0 = w.q0 + static_cast<int>(rank) * kTileQ, part = 0;
+            if (p.q_rows_per_part > 0) {  // a 128-row tile never straddles two parts
+              part = min(s0 / p.q_rows_per_part, kMaxParts - 1);
+              s0 -= part * p.q_rows_per_part;
+            }
+            if (leader_cta) mbar_expect_tx(&q_full[qb], 2 * kQBytes);
+            const BoxCoords c(p.q_pos, w.h, w.b);
+            c.load(sQ + qb * kQBytes, &qmaps.m[part], b_qf + qb * 8, 0, s0);
+            c.load(sQ + qb * kQBytes + kQBytes / 2, &qmaps.m[part], b_qf + qb * 8, 64, s0);
           }
-          if (leader_cta) mbar_expect_tx(&q_full[qb], 2 * kQBytes);
-          const BoxCoords c(p.q_pos, w.h, w.b);
-          c.load(sQ + qb * kQBytes, &qmaps.m[part], b_qf + qb * 8, 0, s0);
-          c.load(sQ + qb * kQBytes + kQBytes / 2, &qmaps.m[part], b_qf + qb * 8, 64, s0);
+          const BoxCoords c(p.k_pos, w.h, w.b);
+          int s0 = w.jb * kTileKV + static_cast<int>(rank) * (kTileKV / 2);
+          for (int j = 0; j < w.nkv; ++j, ++t, s0 += kTileKV) {
+            const uint32_t st = t & (kRing - 1);
+            if (!mbar_wait(&k_empty[st], ((t / kRing) & 1) ^ 1, abort_flag)) goto producer_done;
+            if (leader_cta) mbar_expect_tx(&k_full[st], 2 * kKBytes);
+            c.load(sK + st * kKBytes, &tmap_k, b_kf + st * 8, 0, s0);
+            c.load(sK + st * kKBytes + kKBytes / 2, &tmap_k, b_kf + st * 8, 64, s0);
+          }
         }
-        const BoxCoords c(p.k_pos, w.h, w.b);
-        int s0 = w.jb * kTileKV + static_cast<int>(rank) * (kTileKV / 2);
-        for (int j = 0; j < w.nkv; ++j, ++t, s0 += kTileKV) {
-          const uint32_t st = t & (kRing - 1);
-          if (!mbar_wait(&k_empty[st], ((t / kRing) & 1) ^ 1, abort_flag)) goto producer_done;
-          if (leader_cta) mbar_expect_tx(&k_full[st], 2 * kKBytes);
-          c.load(sK + st * kKBytes, &tmap_k, b_kf + st * 8, 0, s0);
-          c.load(sK + st * kKBytes + kKBytes / 2, &tmap_k, b_kf + st * 8, 64, s0);
+        grid_release();  // a few key tiles before this CTA is done
+      }
+    producer_done:;
+    } else if (warp == kTmaVWarp) {
+      // ------------------------------------------------------------ TMA producer of V
+      if (lane == 0) {
+        const uint32_t b_vf = mapa_u32(smem_u32(v_full), 0);
+        uint32_t t = 0;
+        for (int u = unit0; u < p.n_units; u += n_pairs_grid) {
+          const AttnUnit w = attn_unit<SPLIT>(p, u);
+          const BoxCoords c(p.v_pos, w.h, w.b);
+          int s0 = w.jb * kTileKV;
+          for (int j = 0; j < w.nkv; ++j, ++t, s0 += kTileKV) {
+            const uint32_t st = t & (kRing - 1);
+            if (!mbar_wait(&v_empty[st], ((t / kRing) & 1) ^ 1, abort_flag)) goto v_producer_done;
+            if (leader_cta) mbar_expect_tx(&v_full[st], 2 * kVBytes);
+            c.load(sV + st * kVBytes, &tmap_v, b_vf + st * 8, static_cast<int>(rank) * 64, s0);
+          }
         }
       }
-      grid_release();  // a few key tiles before this CTA is done
-    }
-  producer_done:;
-  } else if (warp == kTmaVWarp) {
-    // ------------------------------------------------------------ TMA producer of V
-    if (lane == 0) {
-      const uint32_t b_vf = mapa_u32(smem_u32(v_full), 0);
-      uint32_t t = 0;
-      for (int u = unit0; u < p.n_units; u += n_pairs_grid) {
-        const AttnUnit w = attn_unit<SPLIT>(p, u);
-        const BoxCoords c(p.v_pos, w.h, w.b);
-        int s0 = w.jb * kTileKV;
-        for (int j = 0; j < w.nkv; ++j, ++t, s0 += kTileKV) {
-          const uint32_t st = t & (kRing - 1);
-          if (!mbar_wait(&v_empty[st], ((t / kRing) & 1) ^ 1, abort_flag)) goto v_producer_done;
-          if (leader_cta) mbar_expect_tx(&v_full[st], 2 * kVBytes);
-          c.load(sV + st * kVBytes, &tmap_v, b_vf + st * 8, static_cast<int>(rank) * 64, s0);
-        }
-      }
-    }
-  v_producer_done:;
-  } else if (warp == kMmaWarp) {
-    // -------------------------------------------------------------- MMA issuer
-    if (leader_cta) {
-      constexpr uint32_t idesc_qk = make_idesc(DFMT_F32, FMT_BF16, FMT_BF16, 0, 0, 256, 128);
-      constexpr uint32_t idesc_pv = make_idesc(DFMT_F32, FMT_BF16, FMT_BF16, 0, 1, 256, 128);
-      // Every descriptor is the low word of a base (the address field, in 16-byte units, never carries out of it) plus an
-      // offset, under one constant high word.
-      const uint64_t q_desc0 = make_desc_k_sw128(smem_u32(sQ));
-      const uint32_t hi = static_cast<uint32_t>(q_desc0 >> 32), q_lo = static_cast<uint32_t>(q_desc0),
-                     k_lo = static_cast<uint32_t>(make_desc_k_sw128(smem_u32(sK))),
-                     v_lo = static_cast<uint32_t>(make_desc_mn_sw128(smem_u32(sV), kVBytes, 1024));  // one 64-column chunk
-      auto desc = [&](uint32_t l) { return (static_cast<uint64_t>(hi) << 32) | l; };
-      const uint32_t b_qf = smem_u32(q_full), b_qe = smem_u32(q_empty), b_kf = smem_u32(k_full), b_ke = smem_u32(k_empty),
-                     b_vf = smem_u32(v_full), b_ve = smem_u32(v_empty), b_sf = smem_u32(s_full), b_pf = smem_u32(p_full), b_of = smem_u32(o_full), b_oe = smem_u32(o_empty);
-      // The score MMAs run three tiles (across items) ahead of the P.V ones: the first three steps issue scores only.
-      // A satisfied wait costs this warp about 100 cycles, most of it the latency of the poll, so the barriers of a step
-      // are polled together.
-      int qk_u = unit0, qk_left = qk_u < p.n_units ? attn_unit<SPLIT>(p, qk_u).nkv : 0;
-      int u = unit0, left = qk_left;
-      uint32_t qk_n = 0, n = 0, kt = 0, vt = 0, sb = 0, pph = 1;  // items and tiles so far; score tile; its P phase
-      bool q_new = true, o_new = true;
-      int lead = kGroups;
-      while (u < p.n_units) {
-        const bool qk = qk_u < p.n_units;
-        const uint32_t kst = kt & (kRing - 1), vst = vt & (kRing - 1), qb = qk_n & 1;
-        if (qk && q_new && !mbar_wait_warp<false>(b_qf + qb * 8, (qk_n >> 1) & 1, abort_flag)) goto mma_done;
-        const uint32_t k_ok = mbar_peek<false>(b_kf + kst * 8, (kt / kRing) & 1);
-        if (lead > 0) {
-          --lead;
-          if (qk && !mbar_wait_warp<false>(b_kf + kst * 8, (kt / kRing) & 1, abort_flag)) goto mma_done;
-        } else {
-          const uint32_t v_ok = mbar_peek<false>(b_vf + vst * 8, (vt / kRing) & 1);
-          const uint32_t p_ok = mbar_peek<true>(b_pf + sb * 8, pph);
-          if (!__all_sync(0xffffffffu, (k_ok & v_ok & p_ok) != 0)) {
+    v_producer_done:;
+    } else if (warp == kMmaWarp) {
+      // -------------------------------------------------------------- MMA issuer
+      if (leader_cta) {
+        constexpr uint32_t idesc_qk = make_idesc(DFMT_F32, FMT_BF16, FMT_BF16, 0, 0, 256, 128);
+        constexpr uint32_t idesc_pv = make_idesc(DFMT_F32, FMT_BF16, FMT_BF16, 0, 1, 256, 128);
+        // Every descriptor is the low word of a base (the address field, in 16-byte units, never carries out of it) plus an
+        // offset, under one constant high word.
+        const uint64_t q_desc0 = make_desc_k_sw128(smem_u32(sQ));
+        const uint32_t hi = static_cast<uint32_t>(q_desc0 >> 32), q_lo = static_cast<uint32_t>(q_desc0),
+                       k_lo = static_cast<uint32_t>(make_desc_k_sw128(smem_u32(sK))),
+                       v_lo = static_cast<uint32_t>(make_desc_mn_sw128(smem_u32(sV), kVBytes, 1024));  // one 64-column chunk
+        auto desc = [&](uint32_t l) { return (static_cast<uint64_t>(hi) << 32) | l; };
+        const uint32_t b_qf = smem_u32(q_full), b_qe = smem_u32(q_empty), b_kf = smem_u32(k_full), b_ke = smem_u32(k_empty),
+                       b_vf = smem_u32(v_full), b_ve = smem_u32(v_empty), b_sf = smem_u32(s_full), b_pf = smem_u32(p_full), b_of = smem_u32(o_full), b_oe = smem_u32(o_empty);
+        // The score MMAs run three tiles (across items) ahead of the P.V ones: the first three steps issue scores only.
+        // A satisfied wait costs this warp about 100 cycles, most of it the latency of the poll, so the barriers of a step
+        // are polled together.
+        int qk_u = unit0, qk_left = qk_u < p.n_units ? attn_unit<SPLIT>(p, qk_u).nkv : 0;
+        int u = unit0, left = qk_left;
+        uint32_t qk_n = 0, n = 0, kt = 0, vt = 0, sb = 0, pph = 1;  // items and tiles so far; score tile; its P phase
+        bool q_new = true, o_new = true;
+        int lead = kGroups;
+        while (u < p.n_units) {
+          const bool qk = qk_u < p.n_units;
+          const uint32_t kst = kt & (kRing - 1), vst = vt & (kRing - 1), qb = qk_n & 1;
+          if (qk && q_new && !mbar_wait_warp<false>(b_qf + qb * 8, (qk_n >> 1) & 1, abort_flag)) goto mma_done;
+          const uint32_t k_ok = mbar_peek<false>(b_kf + kst * 8, (kt / kRing) & 1);
+          if (lead > 0) {
+            --lead;
             if (qk && !mbar_wait_warp<false>(b_kf + kst * 8, (kt / kRing) & 1, abort_flag)) goto mma_done;
-            if (!mbar_wait_warp<false>(b_vf + vst * 8, (vt / kRing) & 1, abort_flag)) goto mma_done;
-            if (!mbar_wait_warp<true>(b_pf + sb * 8, pph, abort_flag)) goto mma_done;
-          }
-          // the epilogue of the item before has read O out
-          if (o_new && !mbar_wait_warp<true>(b_oe, (n & 1) ^ 1, abort_flag)) goto mma_done;
-          const uint32_t b_lo = v_lo + vst * (kVBytes >> 4), a = sb * 128;
-          tc_fence_after();
-          if (elect_one()) {
+          } else {
+            const uint32_t v_ok = mbar_peek<false>(b_vf + vst * 8, (vt / kRing) & 1);
+            const uint32_t p_ok = mbar_peek<true>(b_pf + sb * 8, pph);
+            if (!__all_sync(0xffffffffu, (k_ok & v_ok & p_ok) != 0)) {
+              if (qk && !mbar_wait_warp<false>(b_kf + kst * 8, (kt / kRing) & 1, abort_flag)) goto mma_done;
+              if (!mbar_wait_warp<false>(b_vf + vst * 8, (vt / kRing) & 1, abort_flag)) goto mma_done;
+              if (!mbar_wait_warp<true>(b_pf + sb * 8, pph, abort_flag)) goto mma_done;
+            }
+            // the epilogue of the item before has read O out
+            if (o_new && !mbar_wait_warp<true>(b_oe, (n & 1) ^ 1, abort_flag)) goto mma_done;
+            const uint32_t b_lo = v_lo + vst * (kVBytes >> 4), a = sb * 128;
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)  // 16 keys per instruction = 16 rows of 128 bytes of the V tile, 8 columns of P
-              mma_f16_pair_ts(kTmemO, a + kk * 8, desc(b_lo + kk * 128u), idesc_pv, (!o_new || kk > 0) ? 1u : 0u);
-            tc_commit_pair(b_ve + vst * 8);
-            if (left == 1) tc_commit_pair(b_of);
+              for (int kk = 0; kk < 8; ++kk)  // 16 keys per instruction = 16 rows of 128 bytes of the V tile, 8 columns of P
+                mma_f16_pair_ts(kTmemO, a + kk * 8, desc(b_lo + kk * 128u), idesc_pv, (!o_new || kk > 0) ? 1u : 0u);
+              tc_commit_pair(b_ve + vst * 8);
+              if (left == 1) tc_commit_pair(b_of);
+            }
+            __syncwarp();
+            ++vt;
+            o_new = --left == 0;
+            if (o_new) {
+              ++n;
+              u += n_pairs_grid;
+              if (u < p.n_units) left = attn_unit<SPLIT>(p, u).nkv;
+            }
           }
-          __syncwarp();
-          ++vt;
-          o_new = --left == 0;
-          if (o_new) {
-            ++n;
-            u += n_pairs_grid;
-            if (u < p.n_units) left = attn_unit<SPLIT>(p, u).nkv;
-          }
-        }
-        // scores of the next tile, into the columns whose probabilities the MMAs above have just consumed
-        if (qk) {
-          tc_fence_after();
-          const uint32_t a_lo = q_lo + qb * (kQBytes >> 4), b_lo = k_lo + kst * (kKBytes >> 4);
-          if (elect_one()) {
+          // scores of the next tile, into the columns whose probabilities the MMAs above have just consumed
+          if (qk) {
+            tc_fence_after();
+            const uint32_t a_lo = q_lo + qb * (kQBytes >> 4), b_lo = k_lo + kst * (kKBytes >> 4);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-              mma_f16_pair_ss(sb * 128, desc(a_lo + ((kk >> 2) * (kQBytes / 2 >> 4) + 2 * (kk & 3))),
-                              desc(b_lo + ((kk >> 2) * (kKBytes / 2 >> 4) + 2 * (kk & 3))), idesc_qk, kk > 0 ? 1u : 0u);
-            tc_commit_pair(b_sf + sb * 8);
-            tc_commit_pair(b_ke + kst * 8);
-            if (qk_left == 1) tc_commit_pair(b_qe + qb * 8);
+              for (int kk = 0; kk < 8; ++kk)
+                mma_f16_pair_ss(sb * 128, desc(a_lo + ((kk >> 2) * (kQBytes / 2 >> 4) + 2 * (kk & 3))),
+                                desc(b_lo + ((kk >> 2) * (kKBytes / 2 >> 4) + 2 * (kk & 3))), idesc_qk, kk > 0 ? 1u : 0u);
+              tc_commit_pair(b_sf + sb * 8);
+              tc_commit_pair(b_ke + kst * 8);
+              if (qk_left == 1) tc_commit_pair(b_qe + qb * 8);
+            }
+            __syncwarp();
+            ++kt;
+            q_new = --qk_left == 0;
+            if (q_new) {
+              ++qk_n;
+              qk_u += n_pairs_grid;
+              if (qk_u < p.n_units) qk_left = attn_unit<SPLIT>(p, qk_u).nkv;
+            }
           }
-          __syncwarp();
-          ++kt;
-          q_new = --qk_left == 0;
-          if (q_new) {
-            ++qk_n;
-            qk_u += n_pairs_grid;
-            if (qk_u < p.n_units) qk_left = attn_unit<SPLIT>(p, qk_u).nkv;
-          }
+          if (++sb == kGroups) sb = 0, pph ^= 1;
         }
-        if (++sb == kGroups) sb = 0, pph ^= 1;
       }
+    mma_done:;
     }
-  mma_done:;
-  }
   } else if (warp >= kSoftmaxWarp0) {
     // ----------------------------------------------------------------- softmax
     setmaxnreg_inc<kSoftmaxRegs>();

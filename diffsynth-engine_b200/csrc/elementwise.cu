@@ -266,10 +266,10 @@ static int launch_ln_modulate(const void* x, int64_t ld_x, const float* shift, c
                               int M, int D, float eps, cudaStream_t st) {
   const int nv = (D / 8 + kRowThreads - 1) / kRowThreads;
   const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x);
-#define DSB_LN_CASE(NV)                                                                                         \
-  case NV:                                                                                                      \
-    launch_kernel(ln_modulate_kernel<NV, OUT>, M, kRowThreads, 0, st, xp, ld_x, shift, scale, split_row, shift_b,    \
-                       scale_b, y, ld_y, row_scale, M, D, eps);                                  \
+#define DSB_LN_CASE(NV)                                                                                                \
+  case NV:                                                                                                             \
+    launch_kernel(ln_modulate_kernel<NV, OUT>, M, kRowThreads, 0, st, xp, ld_x, shift, scale, split_row, shift_b,      \
+                       scale_b, y, ld_y, row_scale, M, D, eps);                                                        \
     break;
   switch (nv) {
     DSB_LN_CASE(1) DSB_LN_CASE(2) DSB_LN_CASE(3) DSB_LN_CASE(4) DSB_LN_CASE(5) DSB_LN_CASE(6) DSB_LN_CASE(7)
@@ -1266,11 +1266,11 @@ int dsb_rmsnorm_full(const void* x, int64_t ld_x, void* out, int64_t ld_out, int
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
   const float2* rp = reinterpret_cast<const float2*>(rope);
   int grid = 0;
-#define DSB_RMS_CASE(NV)                                                                                          \
-  case NV:                                                                                                        \
-    grid = persistent_grid<rmsnorm_full_rope_kernel<NV>>(kRowThreads, 0, M);                                       \
-    launch_kernel(rmsnorm_full_rope_kernel<NV>, grid, kRowThreads, 0, st, b, ld_x, o, ld_out, out_chunk_cols,     \
-                       out_chunk_stride, M, D, w, rp, rope_row0, eps);                       \
+#define DSB_RMS_CASE(NV)                                                                                               \
+  case NV:                                                                                                             \
+    grid = persistent_grid<rmsnorm_full_rope_kernel<NV>>(kRowThreads, 0, M);                                           \
+    launch_kernel(rmsnorm_full_rope_kernel<NV>, grid, kRowThreads, 0, st, b, ld_x, o, ld_out, out_chunk_cols,          \
+                       out_chunk_stride, M, D, w, rp, rope_row0, eps);                                                 \
     break;
   switch (nv) {
     DSB_RMS_CASE(1) DSB_RMS_CASE(2) DSB_RMS_CASE(3) DSB_RMS_CASE(4) DSB_RMS_CASE(5) DSB_RMS_CASE(6) DSB_RMS_CASE(7)
@@ -1313,21 +1313,21 @@ static int quant_rows_impl(const void* x, int64_t ld_x, int chunk_cols, int64_t 
   uint8_t* yp = reinterpret_cast<uint8_t*>(y);
   if (out_fmt != DSB_FMT_E4M3 && out_fmt != DSB_FMT_INT8) return DSB_ERR_ARG;
   const int nv = (K / 8 + 255) / 256;
-#define DSB_QR_RING(OUT, NV)                                                                                  \
-  {                                                                                                           \
-    constexpr size_t smem = static_cast<size_t>(kRing) * NV * 256 * 16;                                       \
-    DSB_ENSURE_SMEM((quant_rows_ring_kernel<OUT, NV>), static_cast<int>(smem));                               \
-    const int grid = persistent_grid<quant_rows_ring_kernel<OUT, NV>>(256, smem, M);                          \
-    launch_kernel(quant_rows_ring_kernel<OUT, NV>, grid, 256, smem, st, xp, ld_x, chunk_cols, chunk_stride, yp, ld_y,    \
-                                                             row_scale, M, K);                                \
+#define DSB_QR_RING(OUT, NV)                                                                                           \
+  {                                                                                                                    \
+    constexpr size_t smem = static_cast<size_t>(kRing) * NV * 256 * 16;                                                \
+    DSB_ENSURE_SMEM((quant_rows_ring_kernel<OUT, NV>), static_cast<int>(smem));                                        \
+    const int grid = persistent_grid<quant_rows_ring_kernel<OUT, NV>>(256, smem, M);                                   \
+    launch_kernel(quant_rows_ring_kernel<OUT, NV>, grid, 256, smem, st, xp, ld_x, chunk_cols, chunk_stride, yp, ld_y,  \
+                                                             row_scale, M, K);                                         \
   }
-#define DSB_QR_FMT(OUT)                                                                                       \
-  switch (nv) {                                                                                               \
-    case 1: DSB_QR_RING(OUT, 1) break;                                                                        \
-    case 2: DSB_QR_RING(OUT, 2) break;                                                                        \
-    case 3: DSB_QR_RING(OUT, 3) break;                                                                        \
-    case 4: DSB_QR_RING(OUT, 4) break;                                                                        \
-    default:                                                                                                  \
+#define DSB_QR_FMT(OUT)                                                                                                \
+  switch (nv) {                                                                                                        \
+    case 1: DSB_QR_RING(OUT, 1) break;                                                                                 \
+    case 2: DSB_QR_RING(OUT, 2) break;                                                                                 \
+    case 3: DSB_QR_RING(OUT, 3) break;                                                                                 \
+    case 4: DSB_QR_RING(OUT, 4) break;                                                                                 \
+    default:                                                                                                           \
       launch_kernel(quant_rows_kernel<OUT>, M, 256, 0, st, xp, ld_x, chunk_cols, chunk_stride, yp, ld_y, row_scale, M, K); \
   }
   if (out_fmt == DSB_FMT_E4M3) {
@@ -1459,26 +1459,26 @@ static int run_gemv(const void* W, int64_t ld_w, int w_fmt, const void* x, int64
   // Rows per warp: one when the rows are long (4 KB: eight 16-byte loads a lane) and every one of them can have a warp of
   // its own on the device at once, else four.  3072 x 3072 bf16 14.1 us with four, 10.0 with one; shorter rows lose to the
   // extra CTAs' staging of the activations (3072 x 768 e4m3 5.4 us with four, 6.3 with one).
-#define DSB_GEMV_R(F, R, U, WHEN)                                                                                \
-  if (!done && (WHEN)) {                                                                                         \
-    auto kern = gemv_kernel<F, R, U>;                                                                            \
-    DSB_ENSURE_SMEM(kern, 96 * 1024);                                                                            \
-    /* CTAs that fit: what the registers allow, and what the activations leave of 227 KB (1 KB each is reserved) */ \
-    const int occ = resident_ctas<gemv_kernel<F, R, U>>(256);                                                    \
-    const int fit = static_cast<int>((size_t(227) << 10) / (smem + 1024));                                       \
-    const int resident = (occ < fit ? occ : fit) * sm_count();                                                   \
-    const int blocks = (N + 8 * R - 1) / (8 * R);                                                                \
-    if (R == 4 || blocks <= resident) {                                                                          \
-      launch_kernel(kern, dim3(blocks < resident ? blocks : resident, M), 256, smem, st, W, ldb, x, ld_x, x_bf16, \
-                         w_scale, w_scale_stride, bias, y, ld_y, y_bf16, N, K, act_in, act_out, accumulate);     \
-      done = true;                                                                                               \
-    }                                                                                                            \
+#define DSB_GEMV_R(F, R, U, WHEN)                                                                                      \
+  if (!done && (WHEN)) {                                                                                               \
+    auto kern = gemv_kernel<F, R, U>;                                                                                  \
+    DSB_ENSURE_SMEM(kern, 96 * 1024);                                                                                  \
+    /* CTAs that fit: what the registers allow, and what the activations leave of 227 KB (1 KB each is reserved) */    \
+    const int occ = resident_ctas<gemv_kernel<F, R, U>>(256);                                                          \
+    const int fit = static_cast<int>((size_t(227) << 10) / (smem + 1024));                                             \
+    const int resident = (occ < fit ? occ : fit) * sm_count();                                                         \
+    const int blocks = (N + 8 * R - 1) / (8 * R);                                                                      \
+    if (R == 4 || blocks <= resident) {                                                                                \
+      launch_kernel(kern, dim3(blocks < resident ? blocks : resident, M), 256, smem, st, W, ldb, x, ld_x, x_bf16,      \
+                         w_scale, w_scale_stride, bias, y, ld_y, y_bf16, N, K, act_in, act_out, accumulate);           \
+      done = true;                                                                                                     \
+    }                                                                                                                  \
   }
-#define DSB_GEMV(F)                                            \
-  {                                                            \
-    bool done = false;                                         \
-    DSB_GEMV_R(F, 1, 6, static_cast<int64_t>(K) * esz >= 4096) \
-    DSB_GEMV_R(F, 4, 1, true)                                  \
+#define DSB_GEMV(F)                                                                                                    \
+  {                                                                                                                    \
+    bool done = false;                                                                                                 \
+    DSB_GEMV_R(F, 1, 6, static_cast<int64_t>(K) * esz >= 4096)                                                         \
+    DSB_GEMV_R(F, 4, 1, true)                                                                                          \
   }
   if (w_fmt == DSB_FMT_BF16) DSB_GEMV(0)
   else if (w_fmt == DSB_FMT_E4M3) DSB_GEMV(1)
