@@ -624,20 +624,22 @@ static int launch_group(GemmGroup& grp, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }
 
-// Tile width: 256 columns unless that leaves SMs idle that 128-wide tiles would fill.
+// Tile width, by the rounds of tiles that each choice needs.  A 256 x 256 tile of a CTA pair (more than 256 rows) counts 1; a
+// 128 x 128 tile, a quarter of its work on half its SMs, counts 0.7 and not 0.5, because its operand reads fill the
+// shared-memory port; a 128 x 256 tile of one CTA counts 1.2.  Measured, FP8 with bias, 128- against 256-wide, us:
+// 512 x 3072 -> 3072 10.6 / 13.9 (0.7 against 1 round), -> 9216 18.6 / 15.7 (1.4 / 1), -> 12288 25.3 / 23.1 (2.1 / 2),
+// 300 x 3072 -> 12288 18.5 / 22.7 (1.4 / 2), 200 x 3072 -> 21504 26.1 / 29.6 (2.1 / 2.4), 2048 x 5120 -> 5120 53.0 / 46.3
+// (3.5 / 3), 4095 x 5120 -> 5120 97.3 / 78.9 (6.3 / 5); bf16 183 / 152 for the last.
 static int pick_block_n(int M, int N) {
-  const int tm = (M + kBlockM - 1) / kBlockM;
-  const int t256 = tm * ((N + 255) / 256);
-  const int t128 = tm * ((N + 127) / 128);
-  const int sms = sm_count();
   if (N <= 128) return 128;
-  if (t256 >= sms) {
-    // compare the waves each choice needs, counting a 128-wide tile as half the work
-    const double w256 = static_cast<double>((t256 + sms - 1) / sms);
-    const double w128 = 0.5 * static_cast<double>((t128 + sms - 1) / sms);
-    return (w128 < w256 * 0.92) ? 128 : 256;
-  }
-  return 128;
+  const int64_t sms = sm_count(), rows128 = (M + kBlockM - 1) / kBlockM;
+  const bool pair = M > 256 && N >= 256;
+  const int64_t t256 = (pair ? (M + 2 * kBlockM - 1) / (2 * kBlockM) : rows128) * ((N + 255) / 256);
+  const int64_t t128 = rows128 * ((N + 127) / 128);
+  const int64_t units = pair ? sms / 2 : sms;
+  const double c256 = static_cast<double>((t256 + units - 1) / units) * (pair ? 1.0 : 1.2);
+  const double c128 = static_cast<double>((t128 + sms - 1) / sms) * 0.7;
+  return c128 < c256 ? 128 : 256;
 }
 
 }  // namespace dsb
