@@ -428,6 +428,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     const uint32_t bar_remote = mapa_u32(smem_u32(&p_full[grp]), 0);
     uint32_t sph = 0;
     int g = 0, n = 0, jj = grp;  // tiles of this pair before the item; items before; my next tile inside the item
+    // A wait that runs out is noted here and the lane goes on (with whatever it reads) up to the vote below, so that a warp
+    // gives up as a whole: a lane that left by itself would let the others' votes and TMEM accesses wait for it.
+    bool alive = true;
     for (int u = unit0; u < p.n_units; u += n_pairs_grid, ++n) {
       const AttnUnit w = attn_unit<SPLIT>(p, u);
       float m_ref = 0.f;      // the reference of my last tile
@@ -440,20 +443,21 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         uint32_t a[16], b[16], pk[16];
         // The tile's reference is settled before its scores are there, from what the thread knows of its earlier tiles and
         // from the reference of the tile before (of the item before, for the first tile, which only keeps the order).
-        float m_prev;
-        if (!ref_read(slot, t, &m_prev, abort_flag)) goto softmax_done;
+        float m_prev = 0.f;
+        alive = ref_read(slot, t, &m_prev, abort_flag) && alive;
         const bool move = jj > 0 && run > m_prev + 8.0f;
         float m_new = move ? ceilf(run) : m_prev;
         if (jj > 0) ref_publish(slot, t + 1, m_new);
-        const bool any_move = __any_sync(0xffffffffu, move);
-        if (!mbar_wait(&s_full[grp], sph, abort_flag)) goto softmax_done;
+        const bool any_move = __any_sync(0xffffffffu, move || !alive);
+        if (any_move && __any_sync(0xffffffffu, !alive)) goto softmax_done;
+        alive = mbar_wait(&s_full[grp], sph, abort_flag);
         sph ^= 1;
         tc_fence_after();
         if (any_move) {
           // O (tiles before this one) is brought to the new reference once P.V of the tile before has been added to it.
           // Only now: S of this tile implies P.V of three tiles before, without which the parity of the V stage's barrier,
           // which comes round every four tiles, could be read one round early.
-          if (!mbar_wait(&v_empty[(t - 1) & (kRing - 1)], ((t - 1) / kRing) & 1, abort_flag)) goto softmax_done;
+          alive = mbar_wait(&v_empty[(t - 1) & (kRing - 1)], ((t - 1) / kRing) & 1, abort_flag) && alive;
           tc_fence_after();
           const float alpha = pow2_down(m_prev, m_new);
 #pragma unroll 1
@@ -560,12 +564,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     int n = 0;
     for (int u = unit0; u < p.n_units; u += n_pairs_grid, ++n) {
       const AttnUnit w = attn_unit<SPLIT>(p, u);
-      if (!mbar_wait(&l_full[n & (kSumSlots - 1)], (n / kSumSlots) & 1, abort_flag)) break;
+      if (!mbar_wait_all(&l_full[n & (kSumSlots - 1)], (n / kSumSlots) & 1, abort_flag)) break;
       const float2* sm = sums + (n & (kSumSlots - 1)) * kGroups * kTileQ + row;
       const float2 l0 = sm[0], l1 = sm[kTileQ], l2 = sm[2 * kTileQ];
       const float m = fmaxf(l0.y, fmaxf(l1.y, l2.y));  // the reference of the last tile, which O is relative to
       const float l = l0.x * pow2_down(l0.y, m) + l1.x * pow2_down(l1.y, m) + l2.x * pow2_down(l2.y, m);
-      if (!mbar_wait(o_full, n & 1, abort_flag)) break;
+      if (!mbar_wait_all(o_full, n & 1, abort_flag)) break;
       tc_fence_after();
       auto release = [&]() {  // O has been read out: the next item's first P.V may overwrite it
         tc_fence_before();

@@ -129,6 +129,12 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_wait_limit(bar, parity, abort_flag, kWaitLimitCycles);
 }
+// For a warp whose next steps name all of its lanes (votes, shuffles, tcgen05.ld/st): every lane waits, and all of them go
+// on or all of them give up.  A lane that left by itself would let the others wait for it without a limit.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                              long long limit_cycles = kWaitLimitCycles) {
+  return __all_sync(0xffffffffu, mbar_wait_limit(bar, parity, abort_flag, limit_cycles));
+}
 
 // Latency-critical variant: polls with the non-suspending test_wait, so the waiter notices the phase flip within a
 // few cycles instead of after try_wait's suspend window (measured in the attention kernel: ~285 cycles from the last

@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       // the row's activation scale is fetched before the wait as well
       const float rs = (ep.row_scale && m < M) ? __ldg(ep.row_scale + m) : 1.0f;
       const float rs_t = (ep.col_scale && !ep.col_scale_stride) ? rs * __ldg(ep.col_scale) : rs;  // per-tensor scale folded in
-      if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag)) break;
+      if (!mbar_wait_all(&tmem_full[acc], acc_phase, abort_flag)) break;
       tc_fence_after();
       const bool second = n0 >= ep.split_col;
       const CUtensorMap* tmap_out = second ? &P.o1 : &P.o0;
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             else
               tma_load_2d(sbuf, &P.r, rbar, nb, r0);
           }
-          if (!mbar_wait(rbar, rphase, abort_flag)) {
+          if (!mbar_wait_all(rbar, rphase, abort_flag)) {
             alive = false;
             break;
           }

@@ -113,14 +113,17 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const void* __restrict__
 
 // The give-up path of the bounded waits, exercised on purpose: one warp waits on a barrier that nothing ever
 // arrives at, with a short cycle budget; a second warp stands for the other roles of a real kernel, polls the abort
-// flag and leaves when it is raised.  Both meet at the common exit, where the status word is written - the same
-// sequence the GEMM and attention kernels run when a wait of theirs runs out.
-__global__ void __launch_bounds__(64) wait_timeout_selftest_kernel(long long limit_cycles, int* status, int* left) {
-  __shared__ uint64_t bar;
+// flag and leaves when it is raised; a third, of whose lanes half wait for a barrier that does complete, leaves as a whole.
+// All meet at the common exit, where the status word is written - the same sequence the GEMM and attention kernels run when
+// a wait of theirs runs out.
+__global__ void __launch_bounds__(96) wait_timeout_selftest_kernel(long long limit_cycles, int* status, int* left) {
+  __shared__ uint64_t bar, done_bar;
   __shared__ int abort_word;
+  __shared__ int neighbour_left, warp_left;
   volatile int* abort_flag = &abort_word;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
+    mbar_init(&done_bar, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -131,9 +134,15 @@ __global__ void __launch_bounds__(64) wait_timeout_selftest_kernel(long long lim
   } else if (threadIdx.x == 32) {
     // a neighbour role: its own (long) wait on the same barrier ends as soon as the first role has given up
     const bool done = mbar_wait(&bar, 0, abort_flag);
-    if (left) *left = done ? 0 : 1;
+    neighbour_left = done ? 0 : 1;
+  } else if (warp == 2) {
+    if (threadIdx.x == 64) mbar_arrive(&done_bar);
+    const bool go_on = mbar_wait_all((threadIdx.x & 1) ? &bar : &done_bar, 0, abort_flag, limit_cycles);
+    const unsigned gave_up = __ballot_sync(0xffffffffu, !go_on);
+    if (threadIdx.x == 64) warp_left = gave_up == 0xffffffffu ? 1 : 0;
   }
   __syncthreads();
+  if (threadIdx.x == 0 && left) *left = (neighbour_left && warp_left) ? 1 : 0;
   if (threadIdx.x == 0 && *abort_flag && status) atomicCAS(status, 0, DSB_ERR_TIMEOUT);
 }
 
@@ -186,7 +195,7 @@ extern "C" int dsb_rank_barrier(int* const* flags, int n_ranks, int rank, int ep
 
 extern "C" int dsb_selftest_wait_timeout(long long limit_cycles, int* status, int* neighbour_left, void* stream) {
   if (!status || limit_cycles <= 0 || limit_cycles > kWaitLimitCycles) return DSB_ERR_ARG;
-  wait_timeout_selftest_kernel<<<1, 64, 0, reinterpret_cast<cudaStream_t>(stream)>>>(limit_cycles, status,
+  wait_timeout_selftest_kernel<<<1, 96, 0, reinterpret_cast<cudaStream_t>(stream)>>>(limit_cycles, status,
                                                                                       neighbour_left);
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }

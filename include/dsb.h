@@ -52,8 +52,8 @@ int dsb_version(void);
 /* Self-test of the bounded device waits (no counterpart in the reference, which has no device-side waits): a
  * one-CTA kernel in which one role waits, for at most `limit_cycles` SM cycles (<= 2e9), on a barrier nothing ever
  * arrives at, while a second role waits on the same barrier with the library's ordinary one-second budget.  The
- * first role gives up and raises the CTA's abort flag, the second sees the flag and leaves too (`*neighbour_left`
- * = 1), and `*status` becomes DSB_ERR_TIMEOUT - the sequence every kernel of this library follows when a wait of
+ * first role gives up and raises the CTA's abort flag, the second sees the flag and leaves too, and so does, as a whole,
+ * a warp of which only half of the lanes had such a wait (`*neighbour_left` = 1 if both did), and `*status` becomes DSB_ERR_TIMEOUT - the sequence every kernel of this library follows when a wait of
  * its own runs out.  The context stays usable.  `status` must be 0 on entry to observe the result. */
 int dsb_selftest_wait_timeout(long long limit_cycles, int* status, int* neighbour_left, void* stream);
 

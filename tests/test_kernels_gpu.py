@@ -452,6 +452,14 @@ def test_bounded_wait_runs_out_and_reports_timeout(dsb, cuda_dev):
     dsb.ops.check_status(0)
 
 
+@pytest.mark.parametrize("limit_cycles", [20_000, 500_000])
+def test_a_warp_gives_up_as_a_whole(dsb, cuda_dev, limit_cycles):
+    """The self-test's third warp: half of its lanes wait for a barrier that completes, half for one that does not.  All of
+    its lanes leave (``left`` needs that), as a warp must whose next instruction names every lane."""
+    for _ in range(3):
+        assert dsb.ops.selftest_wait_timeout(limit_cycles=limit_cycles) == (dsb._lib.ERR_TIMEOUT, 1)
+
+
 # ------------------------------------------------------------ attention over row ranges in separate buffers
 def test_flash_attn_parts_equals_one_buffer(dsb, cuda_dev):
     """Queries read from three separate buffers (256 rows each, the last one half used) and output rows written to four
