@@ -32,9 +32,15 @@
 // (`mslot`).  The first tile sets it to ceil(row maximum); after that the thread of a tile moves it, before it has
 // looked at the tile, to the largest exponent that it saw in its own earlier tiles, if that is more than 2^8 above.  So
 // the reference trails by up to three tiles, and no maximum sits on the chain above; a tile's entries that exceed it
-// simply give p > 1 (fp32/bf16 have the range), and row sums and O carry the same reference, so the result is exact.
-// Exponents are cut at 2^100 above the reference.  When a reference moves, O is rescaled in place by that thread, between
-// O += P(j-1) V (it waits for it) and O += P(j) V (which needs its own P).
+// simply give p > 1, and row sums and O carry the same reference.  When a reference moves, O is rescaled in place by that
+// thread, between O += P(j-1) V (it waits for it) and O += P(j) V (which needs its own P).
+//
+// Entries that are more than 2^100 above the reference would leave the range of p.  A tile that meets one (its sums tell)
+// goes on against a higher reference of its own: what it has of P and of the row sum is scaled down, and O too before P is
+// handed over.  The tiles behind it, which may have started with the lower reference, learn of that through a second chain
+// (`fin`: one word per warp of rows, written when a tile's P is complete; `fref`: the rows' references, written only when
+// one is above what `mslot` gave), and scale their P down before they hand it over.  So O, P and the sums always agree,
+// however steeply a row climbs, and nothing is cut.
 //
 // m_ref is always an INTEGER (in log2 units): rescaling by 2^(integer) is exact in floating point, so the bf16
 // rounding of a probability does not depend on which reference it was computed against.  The result therefore equals
@@ -67,7 +73,7 @@ constexpr int kKBytes = (kTileKV / 2) * 256;       // 64 keys, two 64-column hal
 constexpr int kVBytes = kTileKV * 128;             // 128 keys, 64 value columns
 constexpr int kBarBytes = 512;
 constexpr int kAttnSmem = kQBufs * kQBytes + kRing * (kKBytes + kVBytes) + kBarBytes + kTileQ * 8 +
-                          kSumSlots * kGroups * kTileQ * 8 + 1024;
+                          kSumSlots * kGroups * kTileQ * 8 + kTileQ * 4 + 1024;
 
 constexpr int kMaxParts = 8;
 constexpr int kWsRow = 132;  // floats per row of a partial result (528 bytes: rows stay 16-byte aligned)
@@ -121,6 +127,27 @@ __device__ __forceinline__ bool ref_read(const unsigned long long* slot, uint32_
   *v = __uint_as_float(static_cast<uint32_t>(w));
   return true;
 }
+// The word that says what O's references are once a tile has been added to it: twice {tile number + 1}, plus one if some row
+// of the warp has a reference above the one handed on in its slot.  Waits (bounded) for the word of the tile before `t`.
+__device__ __forceinline__ bool fin_read(const volatile uint32_t* word, uint32_t t, bool* above, volatile int* abort_flag) {
+  uint32_t w = *word;
+  if ((w ^ (t << 1)) > 1u) {
+    const long long t0 = clock64();
+    uint32_t spins = 0;
+    do {
+      if (((++spins) & 0xffu) == 0) {
+        if (*abort_flag) return false;
+        if (clock64() - t0 > kWaitLimitCycles) {
+          *abort_flag = 1;
+          return false;
+        }
+      }
+      w = *word;
+    } while ((w ^ (t << 1)) > 1u);
+  }
+  *above = (w & 1) != 0;
+  return true;
+}
 
 // Coordinates (s, h, b) in the order of a tensor map, kept in registers: only s changes inside an item.
 struct BoxCoords {
@@ -172,27 +199,44 @@ __device__ __forceinline__ float pow2_down(float from, float to) {
   return __int_as_float(max(0, 127 + static_cast<int>(from - to)) << 23);
 }
 
-// 16 scores -> 16 probabilities (packed bf16) against the reference, and their sum.  CUT: exponents are cut at 100,
-// columns from `valid` on do not exist, and the largest exponent is kept.
-template <bool CUT>
+// 16 scores -> 16 probabilities (packed bf16) against the reference, and their sum.  CHECK: columns from `valid` on do not
+// exist, and the largest exponent is kept - relative to the reference (1), or by itself (2), which costs a product per score
+// and is exact however far the reference is away.
+template <int CHECK>
 __device__ __forceinline__ void exp_pairs(const uint32_t (&a)[16], uint32_t* pk, float2 cs2, float2 nm2, float2 (&sum)[2],
                                           int valid, float* mx) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const float2 x = __ffma2_rn(make_float2(__uint_as_float(a[2 * i]), __uint_as_float(a[2 * i + 1])), cs2, nm2);
-    float2 pp;
-    if constexpr (CUT) {
-      pp = make_float2(fast_exp2(min_nan(x.x, 100.f)), fast_exp2(min_nan(x.y, 100.f)));
-      if (2 * i < valid) *mx = fmaxf(*mx, x.x);
+    const float2 s = make_float2(__uint_as_float(a[2 * i]), __uint_as_float(a[2 * i + 1]));
+    const float2 x = __ffma2_rn(s, cs2, nm2);
+    float2 pp = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+    if constexpr (CHECK != 0) {
+      const float2 e = CHECK == 2 ? __fmul2_rn(s, cs2) : x;
+      if (2 * i < valid) *mx = fmaxf(*mx, e.x);
       else pp.x = 0.f;
-      if (2 * i + 1 < valid) *mx = fmaxf(*mx, x.y);
+      if (2 * i + 1 < valid) *mx = fmaxf(*mx, e.y);
       else pp.y = 0.f;
-    } else {
-      pp = make_float2(fast_exp2(x.x), fast_exp2(x.y));
     }
     sum[i & 1] = __fadd2_rn(sum[i & 1], pp);
     pk[i] = pack_bf16x2(pp.x, pp.y);
   }
+}
+// 16 columns of TMEM that hold fp32 values (BF16: pairs of bf16) times a power of two
+template <bool BF16>
+__device__ __forceinline__ void scale_columns(uint32_t taddr, float f) {
+  uint32_t r[16];
+  tmem_ld16(taddr, r);
+  tc_wait_ld_regs(r);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if constexpr (BF16) {
+      const float2 v = unpack_bf16x2(r[i]);
+      r[i] = pack_bf16x2(v.x * f, v.y * f);
+    } else {
+      r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
+    }
+  }
+  tmem_st16(taddr, r);
 }
 __device__ __forceinline__ void max_chunk(const uint32_t (&a)[32], float (&mx)[4], bool neg) {
   if (!neg) {
@@ -230,8 +274,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   uint64_t* l_full = o_empty + 1;        // kSumSlots
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(l_full + kSumSlots);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile uint32_t* fin = tmem_slot + 2;  // one word per warp of rows (four)
   unsigned long long* mslot = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(bars) + kBarBytes);
   float2* sums = reinterpret_cast<float2*>(mslot + kTileQ);  // [kSumSlots][kGroups][kTileQ] {row sum, its reference}
+  volatile float* fref = reinterpret_cast<volatile float*>(sums + kSumSlots * kGroups * kTileQ);  // per row, see above
 
   // a warp index that the compiler can see to be uniform: the roles' code then keeps its addresses in uniform registers
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -257,6 +303,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     fence_mbar_init();
   }
   if (threadIdx.x < kTileQ) mslot[threadIdx.x] = 0ull;  // sequence 0 = what the first tile expects
+  if (threadIdx.x < 4) fin[threadIdx.x] = 0u;
   if (warp == kTmaWarp && lane == 0) {
     tma_prefetch_desc(&qmaps.m[0]);
     tma_prefetch_desc(&tmap_k);
@@ -434,9 +481,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     for (int u = unit0; u < p.n_units; u += n_pairs_grid, ++n) {
       const AttnUnit w = attn_unit<SPLIT>(p, u);
       float m_ref = 0.f;      // the reference of my last tile
-      float run = -INFINITY;  // largest exponent (score * cs) among my tiles so far
+      float run = -INFINITY;  // bounds the largest exponent (score * cs) among my tiles so far
       float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       bool first = true;
+      int lift_chunk = -1;                    // >= 0: a tile has left the range of p, see behind the loop
+      float o_ref = 0.f, lift_grown = 0.f, lift_sum = 0.f;
       for (; jj < w.nkv; jj += kGroups) {
         const uint32_t t = static_cast<uint32_t>(g + jj);
         const int valid = p.Sk - (w.jb + jj) * kTileKV;  // columns of this tile that exist (all of them if >= 128)
@@ -459,15 +508,16 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           // which comes round every four tiles, could be read one round early.
           alive = mbar_wait(&v_empty[(t - 1) & (kRing - 1)], ((t - 1) / kRing) & 1, abort_flag) && alive;
           tc_fence_after();
-          const float alpha = pow2_down(m_prev, m_new);
-#pragma unroll 1
-          for (int c = 0; c < 8; ++c) {
-            tmem_ld16(t_o + c * 16, pk);
-            tc_wait_ld_regs(pk);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) pk[i] = __float_as_uint(__uint_as_float(pk[i]) * alpha);
-            tmem_st16(t_o + c * 16, pk);
+          float from = m_prev;
+          bool above = false;
+          alive = fin_read(fin + quad, t, &above, abort_flag) && alive;
+          if (above) {
+            __threadfence_block();
+            from = fref[row];
           }
+          const float alpha = pow2_down(from, fmaxf(m_new, from));
+#pragma unroll 1
+          for (int c = 0; c < 8; ++c) scale_columns<false>(t_o + c * 16, alpha);
         }
         if (jj == 0) {
           // first tile: the row maximum must be known before anything is exponentiated
@@ -498,33 +548,35 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         m_ref = m_new;
         const float2 nm2 = make_float2(-m_new, -m_new);
         float grown_sum = 0.f;
-        float grown = -INFINITY;  // a bound on this tile's largest exponent relative to the reference, see below
+        float grown = -INFINITY;  // the two bound this tile's largest exponent relative to the reference, see below
         // Kept as a short loop: three warps per SM sub-partition run it out of step, and the code of a whole unrolled tile
         // does not stay in the instruction caches.
         tmem_ld16(t_s, a);
+        int c = 0;
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (; c < 4; ++c) {
           const uint32_t t_c = t_s + c * 32;
           float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
           tc_wait_ld_regs(a);
           tmem_ld16(t_c + 16, b);
-          exp_pairs<false>(a, pk, cs2, nm2, sum, 0, nullptr);
+          exp_pairs<0>(a, pk, cs2, nm2, sum, 0, nullptr);
           tc_wait_ld_regs(b);
           if (c < 3) tmem_ld16(t_c + 32, a);
-          exp_pairs<false>(b, pk + 8, cs2, nm2, sum, 0, nullptr);
+          exp_pairs<0>(b, pk + 8, cs2, nm2, sum, 0, nullptr);
           // The sum of the chunk's probabilities bounds their maximum from above and, within a factor of 32, from below:
           // that is all the next reference needs, and takes no instruction per score.
           float total = (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
           if (valid < kTileKV || __any_sync(0xffffffffu, !(total <= 1e30f))) {
-            // The last key tile, a score about 2^100 above the reference, or a NaN: once more, with columns masked and
-            // exponents cut at 100 (the chunk's scores are still in TMEM, P has not reached its columns).
+            // The last key tile, a score about 2^100 above the reference, or a NaN: once more, with columns masked and the
+            // largest exponent known (the chunk's scores are still in TMEM, P has not reached its columns).
             sum[0] = sum[1] = make_float2(0.f, 0.f);
             tmem_ld16(t_c, b);
             tc_wait_ld_regs(b);
-            exp_pairs<true>(b, pk, cs2, nm2, sum, valid - c * 32, &grown);
+            exp_pairs<1>(b, pk, cs2, nm2, sum, valid - c * 32, &grown);
             tmem_ld16(t_c + 16, b);
             tc_wait_ld_regs(b);
-            exp_pairs<true>(b, pk + 8, cs2, nm2, sum, valid - c * 32 - 16, &grown);
+            exp_pairs<1>(b, pk + 8, cs2, nm2, sum, valid - c * 32 - 16, &grown);
+            if (__any_sync(0xffffffffu, grown > 100.f)) break;  // on from this chunk below
             total = 0.f;
           }
           grown_sum = fmaxf(grown_sum, total);
@@ -532,17 +584,123 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           ls[1] = __fadd2_rn(ls[1], sum[1]);
           tmem_st16(t_s + c * 16, pk);
         }
+        // In order behind the tile before; on its own path (below) if that one, or this one, has left the range of p.
+        const uint32_t fin_seen = fin[quad];
+        if (__any_sync(0xffffffffu, c < 4 || fin_seen != t << 1)) {
+          bool above = false;
+          alive = fin_read(fin + quad, t, &above, abort_flag) && alive;
+          if (__any_sync(0xffffffffu, c < 4 || (above && jj > 0))) {
+            lift_chunk = c;
+            o_ref = m_new;
+            lift_grown = fminf(grown, 100.f) + m_ref, lift_sum = grown_sum;
+            break;
+          }
+        }
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
+          fin[quad] = (t << 1) + 2;
           if (leader_cta) mbar_arrive(&p_full[grp]);
           else mbar_arrive_remote(bar_remote);
         }
-        // Exponents beyond 2^100 were cut there, so the next reference may only follow them that far: the row then stays
-        // finite and is dominated by that key, as it should be.
         if (grown_sum > 1.f) grown = fmaxf(grown, static_cast<float>((__float_as_int(grown_sum) >> 23) - 126));
-        run = fmaxf(run, fminf(grown, 100.f) + m_ref);
+        run = fmaxf(run, grown + m_ref);
+      }
+      if (lift_chunk >= 0) {
+        // The group's remaining tiles of the item, the first of them from chunk lift_chunk on: every score is looked at before
+        // its P is stored, and the reference of a row is lifted whenever one is more than 2^100 above it.
+        // `o_ref`: O's reference before this tile, if the tiles before have not lifted it.
+        int c = lift_chunk;
+        float grown = lift_grown, grown_sum = lift_sum, m_new = o_ref;
+        for (;;) {
+          const uint32_t t = static_cast<uint32_t>(g + jj);
+          const int valid = p.Sk - (w.jb + jj) * kTileKV;
+          uint32_t b[16], pk[16];
+          tc_wait_st();
+#pragma unroll 1
+          for (; c < 4; ++c) {
+            const uint32_t t_c = t_s + c * 32;
+            for (;;) {
+              float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+              const float2 nm2 = make_float2(-m_ref, -m_ref);
+              tmem_ld16(t_c, b);
+              tc_wait_ld_regs(b);
+              exp_pairs<2>(b, pk, cs2, nm2, sum, valid - c * 32, &grown);
+              tmem_ld16(t_c + 16, b);
+              tc_wait_ld_regs(b);
+              exp_pairs<2>(b, pk + 8, cs2, nm2, sum, valid - c * 32 - 16, &grown);
+              const float m_to = grown > m_ref + 100.f ? ceilf(grown) : m_ref;
+              if (!__any_sync(0xffffffffu, m_to != m_ref)) {
+                ls[0] = __fadd2_rn(ls[0], sum[0]);
+                ls[1] = __fadd2_rn(ls[1], sum[1]);
+                break;
+              }
+              // the chunk once more, and what there is of the tile and of the row sum scaled down
+              const float alpha = pow2_down(m_ref, m_to);
+              ls[0].x *= alpha, ls[0].y *= alpha, ls[1].x *= alpha, ls[1].y *= alpha;
+#pragma unroll 1
+              for (int i = 0; i < c; ++i) scale_columns<true>(t_s + i * 16, alpha);
+              if (m_to != m_ref) grown_sum = 0.f;  // `grown` covers it
+              m_ref = m_to;
+            }
+            tmem_st16(t_s + c * 16, pk);
+            tc_wait_st();
+          }
+          if (grown_sum > 1.f) grown = fmaxf(grown, static_cast<float>((__float_as_int(grown_sum) >> 23) - 126) + m_ref);
+          // O and P of the warp's rows are brought to the higher of their two references.
+          bool above = false;
+          alive = fin_read(fin + quad, t, &above, abort_flag) && alive;
+          if (jj == 0) {
+            o_ref = m_ref;  // the first tile overwrites O
+          } else if (above) {
+            __threadfence_block();
+            o_ref = fmaxf(o_ref, fref[row]);
+          }
+          const float m_to = fmaxf(m_ref, o_ref);
+          if (__any_sync(0xffffffffu, m_to != o_ref)) {
+            alive = mbar_wait(&v_empty[(t - 1) & (kRing - 1)], ((t - 1) / kRing) & 1, abort_flag) && alive;
+            tc_fence_after();
+            const float alpha = pow2_down(o_ref, m_to);
+#pragma unroll 1
+            for (int i = 0; i < 8; ++i) scale_columns<false>(t_o + i * 16, alpha);
+          }
+          if (__any_sync(0xffffffffu, m_to != m_ref)) {
+            const float alpha = pow2_down(m_ref, m_to);
+#pragma unroll 1
+            for (int i = 0; i < 4; ++i) scale_columns<true>(t_s + i * 16, alpha);
+            ls[0].x *= alpha, ls[0].y *= alpha, ls[1].x *= alpha, ls[1].y *= alpha;
+            m_ref = m_to;
+          }
+          tc_wait_st();
+          if (m_to != m_new) grown = fmaxf(grown, m_to + 8.5f);  // the next tile's reference will not be below this one
+          run = fmaxf(run, grown);
+          const bool lifted = __any_sync(0xffffffffu, m_to != m_new);
+          fref[row] = m_to;
+          __threadfence_block();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            fin[quad] = (t << 1) + (lifted ? 3 : 2);
+            if (leader_cta) mbar_arrive(&p_full[grp]);
+            else mbar_arrive_remote(bar_remote);
+          }
+          jj += kGroups;
+          if (jj >= w.nkv) break;
+          o_ref = 0.f;
+          alive = ref_read(slot, t + kGroups, &o_ref, abort_flag) && alive;
+          m_new = run > o_ref + 8.0f ? ceilf(run) : o_ref;
+          ref_publish(slot, t + kGroups + 1, m_new);
+          if (__any_sync(0xffffffffu, !alive)) goto softmax_done;
+          alive = mbar_wait(&s_full[grp], sph, abort_flag);
+          sph ^= 1;
+          tc_fence_after();
+          const float alpha = pow2_down(m_ref, m_new);
+          ls[0].x *= alpha, ls[0].y *= alpha, ls[1].x *= alpha, ls[1].y *= alpha;
+          m_ref = m_new;
+          grown = -INFINITY, grown_sum = 0.f;
+          c = 0;
+        }
       }
       jj -= w.nkv;
       g += w.nkv;
