@@ -62,7 +62,9 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // completed and its writes are visible.  (Returns at once in a kernel that was launched the ordinary way.)
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // ... and allows that for the next kernel when the calling CTA is about to run out of work.  Not earlier: a waiting CTA holds
-// an SM's shared memory, which a kernel of another stream (a collective) may be waiting for.
+// an SM's shared memory, which a kernel of another stream (a collective) may be waiting for.  And not in a kernel that has a
+// CTA per row or per few rows: the end of a CTA says the same, and the instruction holds such a grid to about one CTA per
+// nanosecond (LayerNorm of 32760 rows of 128 columns: 19 us without it, 36 with).
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- mbarrier

@@ -261,7 +261,6 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 6 ? 7 : 4)) ln_modulate_ke
       }
     }
   }
-  grid_release();
 }
 
 template <int OUT>
@@ -360,7 +359,6 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_heads_kernel(__nv_bfloat16* 
   o.x = pack_bf16x2(x0, x1);
   o.y = pack_bf16x2(x2, x3);
   *reinterpret_cast<uint2*>(p) = o;
-  grid_release();
 }
 
 // ------------------------------------------------------ rmsnorm_full_rope
@@ -582,7 +580,6 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const __nv_bfloat16* __
     }
     *reinterpret_cast<uint2*>(yr + vi * 8) = o;
   }
-  grid_release();
 }
 
 // ------------------------------------------------------------- patchify / unpatchify
@@ -641,7 +638,6 @@ __global__ void __launch_bounds__(256) patchify_kernel(const __nv_bfloat16* __re
       }
     }
   }
-  grid_release();
 }
 
 // unpatchify: token rows [tokens, >= C*4] -> latents [C, F, 2*gh, 2*gw].  c_fastest = 1: feature (py*2 + pz)*C + c
