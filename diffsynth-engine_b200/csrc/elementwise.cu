@@ -364,13 +364,19 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_heads_kernel(__nv_bfloat16* 
 // ------------------------------------------------------ rmsnorm_full_rope
 // RMSNorm over the whole row (all heads, width D = H*128) with weight[D],
 // then per-head RoPE (same 64 (cos,sin) pairs for every head of a token).
-// One CTA per row; in place.  rope == nullptr skips the rotation.
+// Persistent CTAs, a row each at a time; in place.  ROPE: the launch has RoPE factors.
 // The output may be "chunked": column c of row m goes to out[(c / chunk_cols) * chunk_stride + m * ld_out +
 // c % chunk_cols] - the per-peer-contiguous send layout of a head/sequence all-to-all ([P][rows][D/P]).
-// Bound by HBM: 4 bytes an element and 512 bytes of factors a row.  32760 x 5120 with RoPE: 162 -> 119 us
-// (5.8 TB/s, 0.88 of the copy rate); 4608 x 3072 18.5 -> 12.4.
-template <int NV>
-__global__ void __launch_bounds__(kRowThreads, (NV <= 3 ? 7 : NV <= 5 ? 5 : 3)) rmsnorm_full_rope_kernel(
+// Bound by HBM: 4 bytes an element and 512 bytes of factors a row.  32760 x 5120 with RoPE, against one row per CTA: 162 ->
+// 109 us (6.3 TB/s, 0.97 of the copy rate); 4608 x 3072 18.5 -> 10.8.  What does not fit the registers of a CTA waits, so the
+// kernel without RoPE is one of its own with as many CTAs per SM as its registers allow without spilling (with the branch
+// at run time: 16000 x 1024 14.7 us instead of 11.9, 32760 x 5120 115 instead of 109).
+constexpr int rms_ctas(int nv, bool rope) {
+  if (rope) return nv <= 3 ? 7 : nv <= 5 ? 5 : 3;
+  return nv == 1 ? 12 : nv == 2 ? 9 : nv == 3 ? 8 : nv <= 5 ? 5 : 4;
+}
+template <int NV, bool ROPE>
+__global__ void __launch_bounds__(kRowThreads, rms_ctas(NV, ROPE)) rmsnorm_full_rope_kernel(
     const __nv_bfloat16* buf, int64_t ld, __nv_bfloat16* out, int64_t ld_out, int chunk_cols, int64_t chunk_stride, int M,
     int D, const float* __restrict__ w, const float2* __restrict__ rope, int rope_row0, float eps) {
   grid_wait();
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 3 ? 7 : NV <= 5 ? 5 : 3)) 
   float4 rot[2] = {make_float4(1.f, 0.f, 1.f, 0.f), make_float4(1.f, 0.f, 1.f, 0.f)};
   auto load = [&](int r) {
     row_load<NV>(raw, buf + static_cast<int64_t>(r) * ld, nvec);
-    if (rope) {
+    if constexpr (ROPE) {
       rot[0] = __ldg(rope_mine + (static_cast<int64_t>(rope_row0) + r) * 32);
       rot[1] = __ldg(rope_mine + (static_cast<int64_t>(rope_row0) + r) * 32 + 1);
     }
@@ -424,7 +430,7 @@ __global__ void __launch_bounds__(kRowThreads, (NV <= 3 ? 7 : NV <= 5 ? 5 : 3)) 
         float2 o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) o[j] = __fmul2_rn(__fmul2_rn(v[i][j], r2), ww[j]);
-        if (rope) {
+        if constexpr (ROPE) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float a = o[j].x, b = o[j].y;
@@ -1267,11 +1273,15 @@ int dsb_rmsnorm_full(const void* x, int64_t ld_x, void* out, int64_t ld_out, int
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
   const float2* rp = reinterpret_cast<const float2*>(rope);
   int grid = 0;
+#define DSB_RMS_LAUNCH(NV, ROPE)                                                                                       \
+  {                                                                                                                    \
+    grid = persistent_grid<rmsnorm_full_rope_kernel<NV, ROPE>>(kRowThreads, 0, M);                                     \
+    launch_kernel(rmsnorm_full_rope_kernel<NV, ROPE>, grid, kRowThreads, 0, st, b, ld_x, o, ld_out, out_chunk_cols,    \
+                  out_chunk_stride, M, D, w, rp, rope_row0, eps);                                                      \
+  }
 #define DSB_RMS_CASE(NV)                                                                                               \
   case NV:                                                                                                             \
-    grid = persistent_grid<rmsnorm_full_rope_kernel<NV>>(kRowThreads, 0, M);                                           \
-    launch_kernel(rmsnorm_full_rope_kernel<NV>, grid, kRowThreads, 0, st, b, ld_x, o, ld_out, out_chunk_cols,          \
-                       out_chunk_stride, M, D, w, rp, rope_row0, eps);                                                 \
+    if (rp) DSB_RMS_LAUNCH(NV, true) else DSB_RMS_LAUNCH(NV, false)                                                    \
     break;
   switch (nv) {
     DSB_RMS_CASE(1) DSB_RMS_CASE(2) DSB_RMS_CASE(3) DSB_RMS_CASE(4) DSB_RMS_CASE(5) DSB_RMS_CASE(6) DSB_RMS_CASE(7)
@@ -1280,6 +1290,7 @@ int dsb_rmsnorm_full(const void* x, int64_t ld_x, void* out, int64_t ld_out, int
       return DSB_ERR_UNSUPPORTED;
   }
 #undef DSB_RMS_CASE
+#undef DSB_RMS_LAUNCH
   return cudaGetLastError() == cudaSuccess ? DSB_OK : DSB_ERR_CUDA;
 }
 
