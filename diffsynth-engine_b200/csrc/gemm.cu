@@ -845,10 +845,11 @@ extern "C" int dsb_linear_rows(const void* x, int64_t ld_x, const void* Wq, int6
                                const float* w_scale, int w_scale_stride, const float* bias, int act, void* work,
                                int64_t work_bytes, void* out, int64_t ld_out, int* status, void* stream) {
   if (w_fmt != DSB_FMT_E4M3 && w_fmt != DSB_FMT_INT8) return DSB_ERR_ARG;
-  if (M < 0 || N < 0 || K <= 0 || (K & 15) || !w_scale || !work || (reinterpret_cast<uintptr_t>(work) & 15u)) return DSB_ERR_ARG;
+  if (M < 0 || N < 0 || K <= 0 || (K & 15)) return DSB_ERR_ARG;
+  if (M == 0 || N == 0) return DSB_OK;  // an empty product needs no scratch
   const int64_t rows_bytes = static_cast<int64_t>(M) * K;  // a multiple of 16: the row scales behind it are aligned
-  if (work_bytes < rows_bytes + static_cast<int64_t>(M) * 4) return DSB_ERR_ARG;
-  if (M == 0 || N == 0) return DSB_OK;
+  if (!w_scale || !work || (reinterpret_cast<uintptr_t>(work) & 15u) || work_bytes < rows_bytes + static_cast<int64_t>(M) * 4)
+    return DSB_ERR_ARG;
   float* row_scale = reinterpret_cast<float*>(static_cast<unsigned char*>(work) + rows_bytes);
   const int rc = dsb_quant_rows(x, ld_x, work, K, row_scale, M, K, w_fmt, stream);
   if (rc != DSB_OK) return rc;

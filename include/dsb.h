@@ -373,7 +373,7 @@ int dsb_pack_quant_weight(const void* W, int64_t ld_w, int src_is_bf16, void* Wq
 /*
  * Quantised Linear in one call: out = act((quantise_rows(x) . Wq^T) * row_scale * w_scale + bias), i.e. dsb_quant_rows
  * followed by dsb_gemm on caller-provided scratch (`work`, 16-byte aligned, at least M*K + 4*M bytes: the 8-bit rows, then
- * their scales).  Arguments as of dsb_linear_static below; no size limit.
+ * their scales; not looked at when M or N is 0).  Arguments as of dsb_linear_static below; no size limit.
  * Replaces the patched F.linear of utils/fp8_linear.py:27-60.
  */
 int dsb_linear_rows(const void* x, int64_t ld_x, const void* Wq, int64_t ld_w, int w_fmt, int M, int N, int K,

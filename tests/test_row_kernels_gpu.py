@@ -83,3 +83,14 @@ def test_patched_linear_equals_its_parts(dsb, cuda_dev, M, fmt, dtype):
                 want = ops.gemm(q, w.data, row_scale=s, col_scale=w.scale, bias=b)
         assert got.dtype == dtype and got.shape == (*x.shape[:-1], 72)
         assert torch.equal(got.reshape(M, 72), want.to(dtype))
+
+
+@pytest.mark.parametrize("fmt", ["e4m3", "int8"])
+def test_linear_rows_of_an_empty_product(dsb, cuda_dev, fmt):
+    """No rows or no columns: nothing to launch, and no scratch either (an empty tensor has no address)."""
+    code = dsb.ops.FMT_E4M3 if fmt == "e4m3" else dsb.ops.FMT_INT8
+    W, scale = dsb.ops.pack_quant_weight(torch.randn(64, 256, device=cuda_dev), code, per_channel=True)
+    x = torch.randn(9, 256, device=cuda_dev).bfloat16()
+    assert dsb.ops.linear_rows(x[:0], W, scale).shape == (0, 64)
+    assert dsb.ops.linear_rows(x, W[:0], scale[:0]).shape == (9, 0)
+    assert dsb.ops.linear_rows(x, W, scale).shape == (9, 64)

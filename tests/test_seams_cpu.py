@@ -262,3 +262,20 @@ def test_gemm_front_end_checks_shapes_and_dtypes_before_any_launch(dsb):
                 bad.get("bias"), bad.get("gate"))
     with pytest.raises(dsb.DsbError):                                   # a split needs 0 < split_col < N
         chk(M, N, torch.zeros(M, N, dtype=bf), torch.zeros(M, N, dtype=bf), N, e4m3_ok=True)
+
+
+def test_linear_rows_checks_its_arguments_without_a_gpu(dsb):
+    """An empty product returns before the scratch is looked at (no rows need none, and an empty tensor has no address);
+    otherwise the scratch must be there, aligned and large enough."""
+    import ctypes
+    lib = dsb._lib.lib()
+    buf = (ctypes.c_char * 4096)()
+    p16 = (ctypes.addressof(buf) + 15) // 16 * 16
+
+    def call(M=4, N=8, K=64, fmt=1, scale=p16, work=p16, size=4 * (64 + 4)):
+        return lib.dsb_linear_rows(p16, K, p16, K, fmt, M, N, K, scale, 0, None, 0, work, size, p16, 8, None, None)
+
+    assert call(M=0, work=None, size=0) == 0 and call(N=0, work=None, size=0) == 0 and call(N=0, scale=None) == 0
+    for bad in (dict(work=None), dict(work=p16 + 4), dict(size=4 * (64 + 4) - 1), dict(scale=None), dict(fmt=0), dict(K=40),
+                dict(M=-1), dict(N=-1), dict(M=0, K=0)):
+        assert call(**bad) == -1, bad
