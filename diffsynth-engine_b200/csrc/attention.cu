@@ -1078,6 +1078,7 @@ extern "C" int dsb_flash_attn_parts(const void* const* q_parts, int n_q_parts, i
 }
 
 extern "C" int64_t dsb_flash_attn_workspace_bytes(void) {
-  // a last wave of fewer than sm_count() items, cut in at most four
-  return static_cast<int64_t>(sm_count()) * 4 * kPairQ * kWsRow * 4;
+  // a last wave is at least one item short of the pairs that run at once, and its items are cut in at most four
+  const int pairs = resident_pairs();
+  return pairs > 1 ? static_cast<int64_t>(pairs - 1) * 4 * kPairQ * kWsRow * 4 : 0;
 }

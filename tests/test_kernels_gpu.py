@@ -596,10 +596,10 @@ def test_flash_attn_e4m3_output_equals_bf16_output_then_cast(dsb, cuda_dev):
 
 
 def test_flash_attn_parts_with_a_split_last_wave(dsb, cuda_dev):
-    """With a workspace, the items of a partly filled last wave (156 items on a 148-SM part: 8 of them) are cut along
-    the keys into two CTAs each and combined afterwards: the result equals the uncut kernel up to the fp32 summation
-    order of the partial outputs (the bf16 probabilities are identical), the ragged key tail stays masked, and rows of
-    the uncut items are bit-identical."""
+    """With a workspace, the items of a partly filled last wave (156 items on 74 CTA pairs: 8 of them) are cut along
+    the keys into two units each and combined afterwards: the result equals the uncut kernel up to the fp32 summation
+    order of the partial outputs (the bf16 probabilities are identical), the ragged key tail stays masked, rows of
+    the uncut items are bit-identical, and the partial results of the cut ones are all that the workspace is used for."""
     H, Sq, Sk = 3, 52 * 256, 2250
     g = torch.Generator().manual_seed(11)
     q = (torch.randn(1, Sq, H, 128, generator=g) * 1.5).bfloat16().to(cuda_dev)
@@ -608,20 +608,23 @@ def test_flash_attn_parts_with_a_split_last_wave(dsb, cuda_dev):
     want = dsb.ops.flash_attn(q, k, v)[0]
     o_rows = Sq // 2
     o_parts = [torch.zeros(o_rows, H, 128, dtype=torch.bfloat16, device=cuda_dev) for _ in range(2)]
-    ws = dsb.ops.flash_attn_workspace(cuda_dev)
+    ws = dsb.ops.flash_attn_workspace(cuda_dev).fill_(0xAB)
     dsb.ops.flash_attn_parts([q[0]], Sq, (H * 128, 128), k, v, o_parts, o_rows, (H * 128, 128), H, Sq, workspace=ws)
     got = torch.cat(o_parts)
     dsb.ops.check_status(0)
     assert O.rel_l2(got.float().cpu(), want.float().cpu()) < 1e-3
-    sms = torch.cuda.get_device_properties(cuda_dev).multi_processor_count
+    pairs = ws.numel() // (4 * 256 * 528) + 1            # items that run at once: the workspace is for one less, cut in four
     items = 52 * H
-    if items > sms and items % sms:                      # which rows were cut: the last items, head-major
-        n_full = items - items % sms
-        same = torch.ones(Sq, H, dtype=torch.bool)
-        for it in range(n_full, items):
-            same[(it % 52) * 256:(it % 52 + 1) * 256, it // 52] = False
-        assert torch.equal(got.cpu()[same], want.cpu()[same])
-        assert not torch.equal(got.cpu()[~same], want.cpu()[~same]) or True   # may coincide; the bound above is the check
+    tail = items % pairs
+    # which rows were cut: the last items, head-major, in two (three ranges of 18 key tiles would be shorter than eight)
+    assert items > pairs and 0 < tail and -(-tail * 2 // pairs) / 2 + 0.05 < 1, "sizes that leave a last wave worth cutting"
+    same = torch.ones(Sq, H, dtype=torch.bool)
+    for it in range(items - tail, items):
+        same[(it % 52) * 256:(it % 52 + 1) * 256, it // 52] = False
+    assert torch.equal(got.cpu()[same], want.cpu()[same])
+    rows = ws.view(-1, 528)
+    assert not (rows[:tail * 2 * 256, :520] == 0xAB).all(dim=1).any()        # 128 columns, the reference and the row sum
+    assert (rows[tail * 2 * 256:] == 0xAB).all()
     # against the exact restatement of the kernel's rounding, on a sample of the cut rows
     rows = slice(Sq - 256, Sq)
     ref = O.attention_bf16_probs(q[:, rows].transpose(1, 2).float().cpu(), k.transpose(1, 2).float().cpu(),

@@ -235,7 +235,9 @@ def test_new_entry_points_reject_bad_arguments_without_a_gpu(dsb):
     # GGUF: unknown block type, K not a multiple of the block size
     assert lib.dsb_dequant_gguf(99, p16, 144, 2, 256, p16, 256, None) == -4            # DSB_ERR_UNSUPPORTED
     assert lib.dsb_dequant_gguf(14, p16, 210, 2, 200, p16, 200, None) == -1
-    assert int(lib.dsb_flash_attn_workspace_bytes()) >= 0 or True                      # needs a device; only that it links
+    # whole wave positions of four key ranges of 256 rows of 528 bytes; none without a device
+    size = int(lib.dsb_flash_attn_workspace_bytes())
+    assert size >= 0 and size % (4 * 256 * 528) == 0 and (size > 0) == torch.cuda.is_available()
 
 
 def test_gemm_front_end_checks_shapes_and_dtypes_before_any_launch(dsb):
