@@ -586,6 +586,34 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   if (threadIdx.x == 0 && *abort_flag && g.p[0].ep.status) atomicCAS(g.p[0].ep.status, 0, DSB_ERR_TIMEOUT);
 }
 
+// CTA pairs of an instantiation that the current device holds at once, asked once per device (GPCs with an odd SM count
+// leave one SM out)
+template <int KIND, int BLOCK_N, bool TABLE, int EPI>
+static int resident_pairs() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = cached[dev].load();
+  if (n > 0) return n;
+  using SM = GemmSmem<BLOCK_N, 2, TABLE>;
+  auto kern = gemm_kernel<KIND, BLOCK_N, 2, TABLE, EPI>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kTotal) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(sm_count() & ~1, 1, 1);
+  cfg.blockDim = dim3(kGemmThreads, 1, 1);
+  cfg.dynamicSmemBytes = SM::kTotal;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = sm_count() / 2;
+  cached[dev].store(n);
+  return n;
+}
+
 template <int KIND, int BLOCK_N, int CTAS, bool TABLE, int EPI>
 static int launch_group(GemmGroup& grp, cudaStream_t st) {
   using SM = GemmSmem<BLOCK_N, CTAS, TABLE>;
@@ -597,27 +625,8 @@ static int launch_group(GemmGroup& grp, cudaStream_t st) {
     const int grid = tiles < sm_count() ? tiles : sm_count();
     if (launch_kernel(kern, grid, kGemmThreads, SM::kTotal, st, grp) != cudaSuccess) return DSB_ERR_CUDA;
   } else {
-    // persistent grid = the CTA pairs the device can hold at once (GPCs with an odd SM count leave one SM out)
-    static int resident_pairs[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DSB_ERR_CUDA;
-    if (resident_pairs[dev] == 0) {
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 2;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.blockDim = dim3(kGemmThreads, 1, 1);
-      cfg.dynamicSmemBytes = SM::kTotal;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      cfg.gridDim = dim3(sm_count() & ~1, 1, 1);
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = sm_count() / 2;
-      resident_pairs[dev] = n;
-    }
-    const int units = resident_pairs[dev];
+    const int units = resident_pairs<KIND, BLOCK_N, TABLE, EPI>();  // the persistent grid
+    if (units <= 0) return DSB_ERR_CUDA;
     if (launch_kernel<2>(kern, (tiles < units ? tiles : units) * CTAS, kGemmThreads, SM::kTotal, st, grp) != cudaSuccess)
       return DSB_ERR_CUDA;
   }
@@ -630,13 +639,14 @@ static int launch_group(GemmGroup& grp, cudaStream_t st) {
 // 512 x 3072 -> 3072 10.6 / 13.9 (0.7 against 1 round), -> 9216 18.6 / 15.7 (1.4 / 1), -> 12288 25.3 / 23.1 (2.1 / 2),
 // 300 x 3072 -> 12288 18.5 / 22.7 (1.4 / 2), 200 x 3072 -> 21504 26.1 / 29.6 (2.1 / 2.4), 2048 x 5120 -> 5120 53.0 / 46.3
 // (3.5 / 3), 4095 x 5120 -> 5120 97.3 / 78.9 (6.3 / 5); bf16 183 / 152 for the last.
-static int pick_block_n(int M, int N) {
+// `pairs`: CTA pairs that run at once.
+static int pick_block_n(int M, int N, int pairs) {
   if (N <= 128) return 128;
   const int64_t sms = sm_count(), rows128 = (M + kBlockM - 1) / kBlockM;
   const bool pair = M > 256 && N >= 256;
   const int64_t t256 = (pair ? (M + 2 * kBlockM - 1) / (2 * kBlockM) : rows128) * ((N + 255) / 256);
   const int64_t t128 = rows128 * ((N + 127) / 128);
-  const int64_t units = pair ? sms / 2 : sms;
+  const int64_t units = pair ? pairs : sms;
   const double c256 = static_cast<double>((t256 + units - 1) / units) * (pair ? 1.0 : 1.2);
   const double c128 = static_cast<double>((t128 + sms - 1) / sms) * 0.7;
   return c128 < c256 ? 128 : 256;
@@ -764,7 +774,13 @@ extern "C" int dsb_gemm_group(const dsb_gemm_args* args, int count, int fmt, int
   for (int i = 0; i < grp.count; ++i)
     any_norm = any_norm || live[i]->nq_w != nullptr || live[i]->out0_fmt == DSB_FMT_E4M3 ||
                (live[i]->out1 && live[i]->out1_fmt == DSB_FMT_E4M3);  // both need a warp's full 128 columns
-  const int bn = any_norm ? 256 : pick_block_n(live[0]->M, live[0]->N);
+  int bn = 256;
+  if (!any_norm) {
+    // (every instantiation fills an SM by itself, so the number of pairs is the same for all)
+    const int pairs = resident_pairs<KIND_F8, 256, true, EPI_PLAIN>();
+    if (pairs <= 0) return DSB_ERR_CUDA;
+    bn = pick_block_n(live[0]->M, live[0]->N, pairs);
+  }
   // CTA pairs (256 x 256 tiles) when the first problem has enough rows to fill them
   const bool pair = bn == 256 && live[0]->M > 256 && live[0]->N >= 256;
   for (int i = 0; i < grp.count; ++i) {
