@@ -41,12 +41,14 @@ class QuantLinearWeight(nn.Parameter):
     __torch_function__ = torch._C._disabled_torch_function_impl
 
     def bias_f32(self, bias):
-        """fp32 copy of the module's bias (the GEMM epilogue adds an fp32 bias); cached per bias tensor."""
+        """fp32 copy of the module's bias (the GEMM epilogue adds an fp32 bias); made again when the bias is another tensor or
+        has been written in place.  The copy keeps the memory that it was made from, so no other tensor can come to lie at
+        that address."""
         if bias is None:
             return None
         key = (bias.data_ptr(), bias._version)
         if self._bias_f32 is None or self._bias_f32[0] != key:
-            self._bias_f32 = (key, bias.detach().float().contiguous())
+            self._bias_f32 = (key, bias.detach().float().contiguous(), bias.detach())
         return self._bias_f32[1]
 
 

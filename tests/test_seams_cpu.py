@@ -281,3 +281,20 @@ def test_linear_rows_checks_its_arguments_without_a_gpu(dsb):
     for bad in (dict(work=None), dict(work=p16 + 4), dict(size=4 * (64 + 4) - 1), dict(scale=None), dict(fmt=0), dict(K=40),
                 dict(M=-1), dict(N=-1), dict(M=0, K=0)):
         assert call(**bad) == -1, bad
+
+
+def test_bias_copy_follows_the_bias(dsb):
+    """The fp32 copy of a Linear's bias is made again for another bias, also one that the allocator would have put where a
+    dropped one lay, and for one that was written in place."""
+    import importlib
+    quant = importlib.import_module("diffsynth_engine_b200.quant")
+    w = quant.QuantLinearWeight(torch.zeros(64, 32, dtype=torch.int8), torch.ones(1), "int8_channel")
+    assert w.bias_f32(None) is None
+    for i in range(200):
+        bias = torch.full((64,), float(i), dtype=torch.bfloat16)
+        assert torch.equal(w.bias_f32(bias), bias.float()), i
+        bias = torch.full((64,), float(i) + 0.5, dtype=torch.bfloat16)      # the one before is dropped here
+        assert torch.equal(w.bias_f32(bias), bias.float()), i
+        bias.add_(1.0)
+        assert torch.equal(w.bias_f32(bias), bias.float())
+        del bias
