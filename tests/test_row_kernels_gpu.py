@@ -36,7 +36,7 @@ def test_rmsnorm_rows(dsb, cuda_dev, M, D, rope):
 
 @pytest.mark.parametrize("N,K", [(1, 16), (7, 256), (33, 3072), (3072, 4080), (3072, 4096), (5120, 5120), (9000, 4608), (20001, 3072)])
 @pytest.mark.parametrize("fmt", ["bf16", "e4m3", "int8"])
-def test_gemv_rows(dsb, cuda_dev, N, K, fmt):
+def test_one_row(dsb, cuda_dev, N, K, fmt):
     g = torch.Generator(device=cuda_dev).manual_seed(N + K)
     W = torch.randn(N, K, generator=g, device=cuda_dev)
     W = {"bf16": lambda t: t.bfloat16(), "e4m3": lambda t: t.to(torch.float8_e4m3fn),
@@ -94,3 +94,31 @@ def test_linear_rows_of_an_empty_product(dsb, cuda_dev, fmt):
     assert dsb.ops.linear_rows(x[:0], W, scale).shape == (0, 64)
     assert dsb.ops.linear_rows(x, W[:0], scale[:0]).shape == (9, 0)
     assert dsb.ops.linear_rows(x, W, scale).shape == (9, 64)
+
+
+@pytest.mark.parametrize("M", [1, 3, 4])
+@pytest.mark.parametrize("N,K", [(1, 16), (7, 2032), (300, 2048), (33, 2064), (72, 4096), (3072, 3072), (260, 5120), (20001, 4608)])
+@pytest.mark.parametrize("fmt", ["bf16", "e4m3", "int8"])
+def test_few_rows_in_one_launch(dsb, cuda_dev, M, N, K, fmt):
+    """``gemv_rows`` at the widths it is for: more than one trip of the activation staging (K > 2048 from bf16 rows, > 4096
+    from fp32 ones), one and four weight rows per warp, several rows, which may be strided and start at any element, and
+    both output types.  Nothing outside the output's rows is written."""
+    g = torch.Generator(device=cuda_dev).manual_seed(M + N + K)
+    W = torch.randn(N, K, generator=g, device=cuda_dev)
+    W = {"bf16": lambda t: t.bfloat16(), "e4m3": lambda t: t.to(torch.float8_e4m3fn),
+         "int8": lambda t: (t * 30).round().clamp(-127, 127).to(torch.int8)}[fmt](W)
+    bias, scale = torch.randn(N, generator=g, device=cuda_dev), torch.rand(N, generator=g, device=cuda_dev) + 0.5
+    base = torch.randn(M, K + 24, generator=g, device=cuda_dev)
+    for x_dtype in (torch.bfloat16, torch.float32):
+        for off in (0, 1, 8, 13):
+            x = base.to(x_dtype)[:, off:off + K]
+            ref = (x.double() @ W.double().t()) * scale.double() + bias.double()
+            for y_dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 2.5e-3)):
+                out = torch.full((M, N + 3), 7.0, dtype=y_dtype, device=cuda_dev)
+                dsb.ops.gemv_rows(W, x, scale, bias, out=out[:, 1:N + 1])
+                assert O.rel_l2(out[:, 1:N + 1].double(), ref) < tol
+                assert (out[:, 0] == 7).all() and (out[:, N + 1:] == 7).all()
+    assert torch.equal(dsb.ops.gemv_rows(W, base.bfloat16()[:, :K], scale, bias),
+                       dsb.ops.gemv_rows(W, base.bfloat16()[:, :K].contiguous(), scale, bias))
+    rows = base[:1, :K].expand(M, K)                          # one row for all of them
+    assert torch.equal(dsb.ops.gemv_rows(W, rows, scale, bias), dsb.ops.gemv_rows(W, rows.contiguous(), scale, bias))
