@@ -103,7 +103,9 @@ def lib():
     return _lib
 
 
-launches = 0  # successful op calls so far (one kernel launch each on the step's path)
+# op calls so far; a call of the step's path is one kernel launch, linear_rows and linear_static (quantiser and GEMM) and
+# flash_attn_parts with a cut last wave are two, so this is a lower bound of the launches
+launches = 0
 
 
 def check(rc: int, what: str):

@@ -360,8 +360,8 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t dfmt, uint32_t afmt, 
 
 enum { KIND_F16 = 0, KIND_F8 = 1, KIND_I8 = 2 };
 
-// The same two forms for an issue loop that the whole warp runs with one elected lane issuing (`leader` from
-// elect_one()), without the disable-output-lane operand.
+// MMA for an issue loop that the whole warp runs, so that descriptors stay warp-uniform: `leader` (from elect_one(), asked
+// once) guards the instruction itself.  No disable-output-lane operand.
 #define DSB_MMA_ELECT(CG, KINDSTR)                                                                              \
   asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"                         \
                " @q tcgen05.mma.cta_group::" CG ".kind::" KINDSTR " [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),    \
@@ -389,11 +389,8 @@ __device__ __forceinline__ void tc_commit_cg2_elect(uint32_t cluster_addr, uint3
       : "memory");
 }
 
-
-// Forms for an issue loop that the WHOLE warp runs (descriptors stay warp-uniform) with one elected lane issuing:
-// `leader` (from elect_one()) guards the instruction.  No disable-output-lane operand.  Measured in the attention
-// kernel: 16 MMAs issue in ~1000 cycles this way against ~1300 from a lane-0-only branch with the lane-mask form.
-// cta_group::2 forms for one thread of the issuing warp (the body of an `if (elect_one())`).
+// cta_group::2 MMAs for one thread of the issuing warp (the body of an `if (elect_one())`): A from shared memory, or from
+// TMEM.
 __device__ __forceinline__ void mma_f16_pair_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                                 uint32_t accumulate) {
   asm volatile(

@@ -40,8 +40,8 @@ __device__ __forceinline__ float row_scale_from_amax(float amax, float qmax) {
 // The row quantiser walks rows with persistent CTAs and keeps the next kRing-1 rows of each CTA in flight while one
 // is processed: thread t copies its own 16-byte vectors (t, t+T, t+2T, ...) of a row into a slot of a shared-memory
 // ring with cp.async and later reads exactly those vectors back itself, so the ring needs no barrier - only
-// cp.async.wait_group.  Measured at 32760 x 5120: 146 -> 107 us (3.4 -> 4.7 TB/s).  The LayerNorm and RMSNorm kernels
-// walk rows the same way but keep only the next row in flight, in registers: see row_load.
+// cp.async.wait_group.  Measured at 32760 x 5120: 146 -> 107 us (3.4 -> 4.7 TB/s).  The RMSNorm kernel walks rows the same
+// way but keeps only the next row in flight, in registers (row_load); the LayerNorm kernel has a CTA per row.
 constexpr int kRing = 4;
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
