@@ -126,9 +126,10 @@ def _adapters(module) -> List[Tuple[float, torch.Tensor, torch.Tensor]]:
 
 
 def _signature(module):
-    return tuple((name, float(l.scale), float(l.alpha), float(l.rank),
-                  (l.up.weight if hasattr(l.up, "weight") else l.up).data_ptr(),
-                  (l.down.weight if hasattr(l.down, "weight") else l.down).data_ptr())
+    def where(side):
+        w = side.weight if hasattr(side, "weight") else side
+        return w.data_ptr(), w._version
+    return tuple((name, float(l.scale), float(l.alpha), float(l.rank), where(l.up), where(l.down))
                  for name, l in module._lora_dict.items())
 
 
@@ -139,7 +140,9 @@ def _fused_forward(self, x):
     w = self.weight
     sig = _signature(self)
     if getattr(w, "_lora_sig", None) != sig:
-        w.lora_ext = build_lora_extension(w.data, w.scale, w.fmt, _adapters(self)) if sig else None
+        # the adapters are held with what was made of them: no others can be put where dropped ones lay
+        w._lora_held = _adapters(self)
+        w.lora_ext = build_lora_extension(w.data, w.scale, w.fmt, w._lora_held) if sig else None
         w._lora_sig = sig
     return F.linear(x, w, self.bias)
 
@@ -166,6 +169,6 @@ def unfuse_lora(module: torch.nn.Module) -> int:
     for sub in module.modules():
         if getattr(type(sub), "_b200_fused_lora", False):
             sub.__class__ = type(sub)._b200_base
-            sub.weight.lora_ext, sub.weight._lora_sig = None, None
+            sub.weight.lora_ext, sub.weight._lora_sig, sub.weight._lora_held = None, None, None
             n += 1
     return n

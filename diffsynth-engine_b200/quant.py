@@ -36,6 +36,7 @@ class QuantLinearWeight(nn.Parameter):
         self._bias_f32 = None
         self.lora_ext = None      # unfused LoRAs riding in the GEMM as extra K columns (lora.fuse_lora)
         self._lora_sig = None
+        self._lora_held = None
         return self
 
     __torch_function__ = torch._C._disabled_torch_function_impl

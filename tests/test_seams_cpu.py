@@ -298,3 +298,29 @@ def test_bias_copy_follows_the_bias(dsb):
     assert torch.equal(w.bias_f32(bias), bias.float())
     bias.add_(1.0)
     assert torch.equal(w.bias_f32(bias), bias.float())
+
+
+def test_fused_adapters_follow_the_modules_adapters(dsb, monkeypatch):
+    """The extension of a weight is made again for other adapters - also ones that lie where dropped ones lay - and for ones
+    that were written in place, and not otherwise."""
+    import importlib
+    quant, lora = (importlib.import_module("diffsynth_engine_b200." + n) for n in ("quant", "lora"))
+    built = []
+    monkeypatch.setattr(lora, "build_lora_extension", lambda w, scale, fmt, ad: built.append([t.clone() for t in ad[0][1:]]))
+    monkeypatch.setattr(torch.nn.functional, "linear", lambda x, w, b: x)
+    module = types.SimpleNamespace(weight=quant.QuantLinearWeight(torch.zeros(64, 32, dtype=torch.int8), torch.ones(1),
+                                                                  "int8_channel"), bias=None, _lora_dict={})
+    for i in range(20):
+        up, down = torch.full((64, 4), float(i)), torch.full((4, 32), float(i))
+        module._lora_dict["a"] = types.SimpleNamespace(scale=1.0, alpha=4, rank=4, up=up, down=down)
+        for _ in range(2):
+            lora._fused_forward(module, torch.zeros(1))
+        assert len(built) == i + 1 and (built[-1][0] == i).all() and (built[-1][1] == i).all()
+        module._lora_dict.clear()
+        del up, down
+    up, down = torch.zeros(64, 4), torch.zeros(4, 32)
+    module._lora_dict["a"] = types.SimpleNamespace(scale=1.0, alpha=4, rank=4, up=up, down=down)
+    lora._fused_forward(module, torch.zeros(1))
+    down.add_(1.0)
+    lora._fused_forward(module, torch.zeros(1))
+    assert len(built) == 22 and (built[-1][1] == 1).all()
