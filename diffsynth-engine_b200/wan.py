@@ -308,12 +308,13 @@ class WanDiTEngine:
             if clip_feature is not None or y is not None:
                 raise ValueError("this model has no image branch (no img_emb / k_img / v_img weights)")
             b["latents"].copy_(x.reshape(b["latents"].shape), non_blocking=True)
-        # the cross-attention keys / values are cached per context: the same tensor object, unmodified since the last
-        # call (a pipeline passes its prompt embedding again at every denoising step), keeps them
-        key = (context.data_ptr(), context._version, tuple(context.shape), str(context.device),
+        # the cross-attention keys / values are cached per context: the same memory, unmodified since the last call (a
+        # pipeline passes its prompt embedding again at every denoising step), keeps them.  The tensors are held meanwhile,
+        # so that no other prompt's embedding can be put where a dropped one lay.
+        key = (context.data_ptr(), context._version, tuple(context.shape), context.stride(), context.dtype, str(context.device),
                None if clip_feature is None else (clip_feature.data_ptr(), clip_feature._version))
         if b.get("ctx_key") != key:
-            b["ctx_key"], b["ctx_valid"] = key, False
+            b["ctx_key"], b["ctx_valid"], b["ctx_held"] = key, False, (context, clip_feature)
             b["context_in"].copy_(context.reshape(b["context_in"].shape), non_blocking=True)
         b["t"].copy_(timestep.reshape(1), non_blocking=True)
 

@@ -74,6 +74,27 @@ def test_wan_image_to_video_engine_matches_oracle(dsb, cuda_dev, fmt):
         eng(x.to(dev), context.to(dev), t.to(dev))       # image-to-video weights without the image inputs
 
 
+def test_another_prompt_is_never_taken_for_a_dropped_one(dsb, cuda_dev):
+    """Keys and values of the prompt are kept from step to step; a prompt embedding that replaces a dropped one, which the
+    allocator would put at the same address, gets its own."""
+    from diffsynth_engine_b200.wan import WanDiTEngine
+    w, x, context, t = _case()
+    eng = WanDiTEngine(dict(w), fmt="bf16", device=cuda_dev, num_layers=2, num_heads=H)
+    x, t = x.to(cuda_dev), t.to(cuda_dev)
+    outs = []
+    for i in range(3):
+        prompt = (context * (1.0 - i)).to(cuda_dev)
+        outs.append(eng(x, prompt, t).clone())
+        assert torch.equal(eng(x, prompt, t), outs[-1])
+        torch.cuda.synchronize()
+        del prompt
+    for i in range(3):
+        fresh = WanDiTEngine(dict(w), fmt="bf16", device=cuda_dev, num_layers=2, num_heads=H)
+        kept = (context * (1.0 - i)).to(cuda_dev)
+        assert torch.equal(fresh(x, kept, t), outs[i])
+    assert not torch.equal(outs[0], outs[1])
+
+
 def test_wan_rope_table_matches_oracle(dsb, cuda_dev):
     from diffsynth_engine_b200.wan import wan_rope_table
     assert torch.equal(wan_rope_table(3, 4, 5, device=cuda_dev).cpu(), O.wan_rope_table(3, 4, 5))
