@@ -331,8 +331,8 @@ def test_flash_attn_peaked_rows(dsb, cuda_dev):
 
 def test_flash_attn_one_key_far_above_the_reference_maximum(dsb, cuda_dev):
     """One key deep in the sequence scores more than 2^100 above everything before it for about half of the rows (and
-    as far below for the rest): the chunk that meets it is redone with clamped exponents, the next tile refreshes
-    the reference maximum, and the rows it dominates return that key's value."""
+    as far below for the rest): the tile that meets it lifts the reference of its rows, and the rows it dominates return
+    that key's value."""
     g = _gen(19)
     H, S = 2, 2048
     q = _bf(torch.randn(1, S, H, 128, generator=g))
